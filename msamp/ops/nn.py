@@ -190,10 +190,10 @@ def gelu(x):
 
 
 # ---------------------------------------------------------------------------------------- attention
-def _attn_entry(d, which):
-    """Native entry point for head size ``d``: the tcgen05 kernels for 128 (``MSAMP_ATTN_IMPL=mma`` keeps the
-    mma.sync kernels, which always serve head size 64)."""
-    tc = d == 128 and os.environ.get('MSAMP_ATTN_IMPL', 'tc') != 'mma'
+def _attn_entry(which):
+    """Native entry point: the tcgen05 kernels (``MSAMP_ATTN_IMPL=mma`` selects the mma.sync kernels, which also serve views
+    with a zero stride)."""
+    tc = os.environ.get('MSAMP_ATTN_IMPL', 'tc') != 'mma'
     return getattr(native.lib(), f'msamp_attention_{"tc_" if tc else ""}{which}')
 
 
@@ -212,7 +212,7 @@ class _AttentionFn(torch.autograd.Function):
         lse = torch.empty((B, nh, S), dtype=torch.float32, device=q.device)
         st = _strides(q) + _strides(k) + _strides(v) + _strides(o) + [0] * 12
         native.check(
-            _attn_entry(d, 'fwd')(
+            _attn_entry('fwd')(
                 native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(o), native.ptr(lse), _i64x24(*st), B, nh, S, d,
                 ctypes.c_float(scale), int(causal), native.stream()
             ), 'attention_fwd'
@@ -236,7 +236,7 @@ class _AttentionFn(torch.autograd.Function):
         delta = torch.empty((B, nh, S), dtype=torch.float32, device=q.device)
         st = _strides(q) + _strides(k) + _strides(v) + _strides(o) + _strides(d_o) + _strides(dq) + _strides(dk) + _strides(dv)
         native.check(
-            _attn_entry(d, 'bwd')(
+            _attn_entry('bwd')(
                 native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(o), native.ptr(lse), native.ptr(d_o), native.ptr(dq),
                 native.ptr(dk), native.ptr(dv), native.ptr(delta), _i64x24(*st), B, nh, S, d, ctypes.c_float(ctx.scale), int(ctx.causal),
                 native.stream()
@@ -259,7 +259,7 @@ class _AttentionPackedFn(torch.autograd.Function):
         lse = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
         st = _strides(q) + _strides(k) + _strides(v) + _strides(o) + [0] * 12
         native.check(
-            _attn_entry(d, 'fwd')(
+            _attn_entry('fwd')(
                 native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(o), native.ptr(lse), _i64x24(*st), B, nh, S, d,
                 ctypes.c_float(scale), int(causal), native.stream()
             ), 'attention_fwd'
@@ -280,7 +280,7 @@ class _AttentionPackedFn(torch.autograd.Function):
         delta = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
         st = _strides(q) + _strides(k) + _strides(v) + _strides(o) + _strides(d_o) + _strides(dq) + _strides(dk) + _strides(dv)
         native.check(
-            _attn_entry(d, 'bwd')(
+            _attn_entry('bwd')(
                 native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(o), native.ptr(lse), native.ptr(d_o), native.ptr(dq),
                 native.ptr(dk), native.ptr(dv), native.ptr(delta), _i64x24(*st), B, nh, S, d, ctypes.c_float(ctx.scale), int(ctx.causal),
                 native.stream()
@@ -301,7 +301,7 @@ def attention_qkv_fwd_raw(qkv, causal=True, scale=None):
         lse = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
         st = _strides(q) + _strides(k) + _strides(v) + _strides(o) + [0] * 12
         native.check(
-            _attn_entry(d, 'fwd')(
+            _attn_entry('fwd')(
                 native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(o), native.ptr(lse), _i64x24(*st), B, nh, S, d,
                 ctypes.c_float(scale), int(causal), native.stream()
             ), 'attention_fwd'
@@ -324,7 +324,7 @@ def attention_qkv_bwd_raw(qkv, o, lse, d_o, causal=True, scale=None):
         delta = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
         st = _strides(q) + _strides(k) + _strides(v) + _strides(o) + _strides(d_o) + _strides(dq) + _strides(dk) + _strides(dv)
         native.check(
-            _attn_entry(d, 'bwd')(
+            _attn_entry('bwd')(
                 native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(o), native.ptr(lse), native.ptr(d_o), native.ptr(dq),
                 native.ptr(dk), native.ptr(dv), native.ptr(delta), _i64x24(*st), B, nh, S, d, ctypes.c_float(scale), int(causal),
                 native.stream()

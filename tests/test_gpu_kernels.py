@@ -550,6 +550,52 @@ def test_attention_kernel_variants(env):
     assert res.returncode == 0 and 'ok' in res.stdout, res.stderr[-2000:]
 
 
+def _rel(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm()).item()
+
+
+# work lists of the persistent kernels: one item, fewer items than SMs (both streams of a CTA share an item), a last wave that
+# is shared (300 = 2 * 148 + 4 items), a last wave with up to two items per CTA, tiles with 1, 2 and 127 rows
+@pytest.mark.parametrize('d', [64, 128])
+@pytest.mark.parametrize('shape', [(1, 1, 1, True), (2, 127, 5, True), (1, 129, 3, False), (1, 128, 149, False), (5, 130, 30, False), (3, 257, 33, True),
+                                   (4, 384, 40, True)])
+def test_attention_work_lists(d, shape):
+    B, S, H, causal = shape
+    torch.manual_seed(1)
+    qkv = torch.randn(B, S, 3, H, d, device=DEV, dtype=torch.bfloat16).requires_grad_()
+    do = torch.randn(B, S, H, d, device=DEV, dtype=torch.bfloat16)
+    o = K.attention_qkv(qkv, causal=causal)
+    o.backward(do)
+    ref_in = qkv.detach().float().requires_grad_()
+    r = _attn_ref(ref_in[:, :, 0], ref_in[:, :, 1], ref_in[:, :, 2], causal)
+    r.backward(do.float())
+    # bf16 roundings of 2^-9: P and the output forward; P or dS, the saved output and the gradient backward
+    assert _rel(o, r) <= 2 * 2**-9
+    if S > 1:    # with one key the gradients of q and k are exactly zero
+        assert _rel(qkv.grad, ref_in.grad) <= 3 * 2**-9
+    assert native.device_status() == 0
+
+
+@pytest.mark.parametrize('d', [64, 128])
+def test_attention_repeated_heads(d):
+    """Views with a zero stride (one K / V head for all query heads), which no tensor map can describe."""
+    torch.manual_seed(2)
+    B, S, H = 2, 200, 4
+    q = torch.randn(B, S, H, d, device=DEV, dtype=torch.bfloat16).requires_grad_()
+    kv = torch.randn(2, B, S, 1, d, device=DEV, dtype=torch.bfloat16)
+    k, v = (t.expand(B, S, H, d).detach().requires_grad_() for t in kv)
+    assert k.stride(2) == 0
+    o = K.attention(q, k, v, causal=True)
+    do = torch.randn_like(o)
+    o.backward(do)
+    leaves = [t.detach().float().requires_grad_() for t in (q, k, v)]
+    r = _attn_ref(*leaves, True)
+    r.backward(do.float())
+    assert _rel(o, r) <= 2 * 2**-9
+    for got, ref in zip((q, k, v), leaves):
+        assert _rel(got.grad, ref.grad) <= 3 * 2**-9
+
+
 def test_cross_entropy():
     torch.manual_seed(0)
     rows, vocab = 300, 50304
