@@ -104,6 +104,33 @@ __device__ __forceinline__ float msamp_compute_scale(float amax, float old_scale
   return exp2f(e);    // exact for integral e
 }
 
+// Two fp32 lanes per instruction (f32x2): the same roundings as the scalar forms at half the issue slots.
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ float2 f2_unpack(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 // amax values are non-negative or +inf, for which the IEEE bit pattern is monotone as an integer.
 __device__ __forceinline__ void atomic_max_nonneg(float* addr, float v) {
   atomicMax(reinterpret_cast<int*>(addr), __float_as_int(v));
@@ -129,6 +156,10 @@ __device__ __forceinline__ float gelu_grad_f(float x) {
   // d/dx [x s(2u)] = s + x * 2 s (1 - s) * du/dx
   return s + 2.0f * x * s * (1.0f - s) * k0 * (1.0f + 3.0f * k1 * x * x);
 }
+
+// The same maximum kept as an integer: |v| as bits (NaN sorts above +inf), two instructions per value.
+__device__ __forceinline__ uint32_t amax_bits(uint32_t m, float v) { return max(m, __float_as_uint(v) & 0x7fffffffu); }
+__device__ __forceinline__ float amax_from_bits(uint32_t m) { return __uint_as_float(min(m, 0x7f800000u)); }
 
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll

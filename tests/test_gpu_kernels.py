@@ -295,6 +295,20 @@ def test_add_to_fp8_bit_exact():
                 assert t.meta.scale.item() == c.meta.scale.item() and t.meta.amax[0].item() == c.meta.amax[0].item()
 
 
+@pytest.mark.parametrize('shape', [(1, 8), (31, 248), (33, 264), (257, 256), (1576, 3072), (5000, 40)])    # rows per CTA, column slabs of 256
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
+def test_cast_colsum_slabs(shape, dtype):
+    torch.manual_seed(0)
+    x = torch.randn(*shape, device=DEV).to(dtype)
+    s, am, cs = torch.tensor(8.0, device=DEV), torch.zeros((), device=DEV), torch.zeros(shape[1], device=DEV)
+    out = cast.cast_to_fp8(x, E5, s, am, colsum_out=cs)
+    assert torch.equal(out.cpu(), cast.cast_to_fp8(x.cpu(), E5, s.cpu()))
+    assert am.item() == x.float().abs().max().item()
+    # fp32 sums of `rows` terms in some order: at most rows * 2^-24 of the sum of magnitudes
+    bound = shape[0] * 2**-24 * x.double().abs().sum(0) + 1e-30
+    assert ((cs.double() - x.double().sum(0)).abs() <= bound).all()
+
+
 def test_fp4_and_sumsq():
     x = (torch.randn(10007, device=DEV) * 3).bfloat16()
     assert torch.equal(arith.fp4_quantize_e2m1(x).cpu(), arith.fp4_quantize_e2m1(x.cpu()))
