@@ -295,6 +295,19 @@ def test_add_to_fp8_bit_exact():
                 assert t.meta.scale.item() == c.meta.scale.item() and t.meta.amax[0].item() == c.meta.amax[0].item()
 
 
+@pytest.mark.parametrize('n', [7, 8, 9, 16 * 256, 148 * 6 * 256 * 16 + 8 * 256 + 5])    # one vector, its neighbours, one and several grid steps
+@pytest.mark.parametrize('offset', [0, 1])    # the byte-wise path of unaligned slices
+def test_add_to_fp8_vector_edges(n, offset):
+    for dt in (torch.float32, torch.bfloat16):
+        t = torch.randn(n + offset, device=DEV).cast(E4)
+        c = t.cpu()
+        other = torch.randn(n + offset, device=DEV).to(dt)
+        arith.add_to_fp8(t.value[offset:], E4, t.meta.scale, t.meta.scale_inv, t.meta.amax[0], other[offset:])
+        arith.add_to_fp8(c.value[offset:], E4, c.meta.scale, c.meta.scale_inv, c.meta.amax[0], other[offset:].cpu())
+        assert torch.equal(t.value.cpu(), c.value)
+        assert t.meta.scale.item() == c.meta.scale.item() and t.meta.amax[0].item() == c.meta.amax[0].item()
+
+
 @pytest.mark.parametrize('shape', [(1, 8), (31, 248), (33, 264), (257, 256), (1576, 3072), (5000, 40)])    # rows per CTA, column slabs of 256
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
 def test_cast_colsum_slabs(shape, dtype):
