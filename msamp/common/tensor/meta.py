@@ -52,7 +52,7 @@ class ScalingMeta:
 
     def is_warmup(self):
         """True until ``window_size`` optimizer steps have been recorded."""
-        return bool(self.amax_counter < self.window_size)
+        return self.amax_counter.item() < self.window_size
 
     def is_in_time_scaling(self):
         """Whether the next cast derives its scale from the tensor being cast."""

@@ -116,10 +116,12 @@ class ModelState:
             return
         for k, v in scaling_metas.items():
             flat = self._flattened_scaling_metas[k]
-            self._check_in_mem(v.scale, flat['scales'])
-            self._check_in_mem(v.scale_inv, flat['scales_inv'])
-            self._check_in_mem(v.amax, flat['amaxs'])
-            self._check_in_mem(v.amax_counter, flat['amax_counters'])
+            for inner, outer in ((v.scale, flat['scales']), (v.scale_inv, flat['scales_inv']), (v.amax, flat['amaxs']),
+                                 (v.amax_counter, flat['amax_counters'])):
+                # addresses are unique over the host and all devices; what is not plainly inside goes to the full check
+                off = inner.data_ptr() - outer.data_ptr()
+                if off < 0 or off + inner.nbytes > outer.nbytes or outer.nbytes == 0:
+                    self._check_in_mem(inner, outer)
 
     def register_scaling_metas(self, model, group=None):
         """Collect ``scaling_metas`` of every submodule of ``model`` and (re)build the flat buffers."""

@@ -21,7 +21,7 @@ _counters = {}
 
 def _counter(device):
     """Zeroed scratch word used by the amax kernel's last-block election (one per device and stream)."""
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
+    key = (device, native.raw_stream() if device.index == torch.cuda.current_device() else torch.cuda.current_stream(device).cuda_stream)
     c = _counters.get(key)
     if c is None:
         c = torch.zeros(1, dtype=torch.int32, device=device)
@@ -46,10 +46,8 @@ def amax(x, out=None):
             out = torch.empty((), dtype=torch.float32, device=x.device)
         x = x.contiguous()
         native.check(
-            native.lib().msamp_amax(
-                native.ptr(x), native.i64(x.numel()), native.dt(x.dtype), native.ptr(out), None, None, ctypes.c_float(0), 0,
-                ctypes.c_float(1), None, native.stream()
-            ), 'amax'
+            native.lib().msamp_amax(x.data_ptr(), x.numel(), native.dt(x.dtype), out.data_ptr(), None, None, 0.0, 0, 1.0, None, native.raw_stream()),
+            'amax'
         )
         return out
     if x.numel() == 0:
@@ -69,9 +67,8 @@ def amax_and_scale(x, amax_out, scale, scale_inv, qtype, margin=0, prescale=1.0)
         x = x.contiguous()
         native.check(
             native.lib().msamp_amax(
-                native.ptr(x), native.i64(x.numel()), native.dt(x.dtype), native.ptr(amax_out), native.ptr(scale),
-                native.ptr(scale_inv), ctypes.c_float(fp_max), int(margin), ctypes.c_float(prescale), native.ptr(_counter(x.device)),
-                native.stream()
+                x.data_ptr(), x.numel(), native.dt(x.dtype), amax_out.data_ptr(), scale.data_ptr(), native.addr(scale_inv), fp_max, int(margin),
+                prescale, _counter(x.device).data_ptr(), native.raw_stream()
             ), 'amax_and_scale'
         )
         return
@@ -113,19 +110,19 @@ def cast_to_fp8(x, qtype, scale, amax_out=None, scale_inv_out=None, amax_in=None
         x = x.contiguous()
         if out is None:
             out = torch.empty(x.shape, dtype=torch.uint8, device=x.device)
-        if colsum_out is not None and (x.shape[1] * x.element_size()) % 16 == 0 and x.data_ptr() % 16 == 0 and out.data_ptr() % 8 == 0:
+        px, pout, addr = x.data_ptr(), out.data_ptr(), native.addr
+        if colsum_out is not None and (x.shape[1] * x.element_size()) % 16 == 0 and px % 16 == 0 and pout % 8 == 0:
             native.check(
                 native.lib().msamp_cast_to_fp8_colsum(
-                    native.ptr(x), x.shape[0], x.shape[1], native.dt(x.dtype), native.ptr(out), native.fmt(qtype), native.ptr(scale),
-                    native.ptr(amax_out), native.ptr(scale_inv_out), native.ptr(colsum_out), native.ptr(amax_in), native.stream()
+                    px, x.shape[0], x.shape[1], native.dt(x.dtype), pout, native.fmt(qtype), scale.data_ptr(), addr(amax_out),
+                    addr(scale_inv_out), colsum_out.data_ptr(), addr(amax_in), native.raw_stream()
                 ), 'cast_to_fp8_colsum'
             )
             return out
         native.check(
             native.lib().msamp_cast_to_fp8_ex(
-                native.ptr(x), native.i64(x.numel()), native.dt(x.dtype), native.ptr(out), native.fmt(qtype), native.ptr(scale),
-                native.ptr(amax_out), native.ptr(scale_inv_out), native.ptr(amax_in), ctypes.c_float(prescale), int(bool(rescale)),
-                1 if act == 'gelu' else 0, native.stream()
+                px, x.numel(), native.dt(x.dtype), pout, native.fmt(qtype), scale.data_ptr(), addr(amax_out), addr(scale_inv_out),
+                addr(amax_in), prescale, int(bool(rescale)), 1 if act == 'gelu' else 0, native.raw_stream()
             ), 'cast_to_fp8'
         )
         if colsum_out is not None:

@@ -46,7 +46,8 @@ def _gelu_tanh_grad(x):
 
 
 def _fix_operand(t):
-    if t.stride(1) != 1 or t.stride(0) % 16 or t.data_ptr() % 16:
+    s = t.stride()
+    if s[1] != 1 or s[0] % 16 or t.data_ptr() % 16:
         t = t.contiguous()
     return t
 
@@ -118,30 +119,16 @@ def gemm_fp8(a, a_qtype, a_scale_inv, b, b_qtype, b_scale_inv, out_dtype, bias=N
             amax_out.zero_()
         if colsum_out is not None:
             colsum_out.zero_()
-        g = _GemmDesc()
-        g.a, g.b, g.d = a.data_ptr(), b.data_ptr(), (out.data_ptr() if out is not None else None)
-        g.colsum = colsum_out.data_ptr() if colsum_out is not None else None
-        g.bias = bias.data_ptr() if bias is not None else None
-        g.residual = residual.data_ptr() if residual is not None else None
-        g.gelu_src = gelu_src.data_ptr() if gelu_src is not None else None
-        g.scale_inv_a, g.scale_inv_b = a_scale_inv.data_ptr(), b_scale_inv.data_ptr()
-        g.amax_out = amax_out.data_ptr() if amax_out is not None else None
-        g.d8 = out8.data_ptr() if out8 is not None else None
-        g.d8_scale = out8_scale.data_ptr() if out8 is not None else None
-        g.d8_scale_inv_out = out8_scale_inv_out.data_ptr() if (out8 is not None and out8_scale_inv_out is not None) else None
-        g.lda, g.ldb, g.ldd = a.stride(0), b.stride(0), (out.stride(0) if out is not None else N)
-        g.ldr = residual.stride(0) if residual is not None else 0
-        g.ldg = gelu_src.stride(0) if gelu_src is not None else 0
-        g.ld8 = out8.stride(0) if out8 is not None else 0
-        g.M, g.N, g.K = M, N, K
-        g.a_fmt, g.b_fmt = native.fmt(a_qtype), native.fmt(b_qtype)
-        g.d8_fmt = native.fmt(out8_qtype) if out8 is not None else 0
-        g.a_mn, g.b_mn = int(bool(a_mn)), int(bool(b_mn))
-        g.out_dtype = native.dt(out_dtype)
-        g.bias_dtype = native.dt(bias.dtype) if bias is not None else 0
-        g.act = 1 if act == 'gelu' else 0
-        g.max_ctas, g.tile = int(max_ctas), int(tile) or _DEFAULT_TILE
-        g.stats = stats.data_ptr() if stats is not None else None
+        addr, has8 = native.addr, out8 is not None
+        g = _GemmDesc(    # in the order of _fields_
+            a.data_ptr(), b.data_ptr(), addr(out), addr(bias), addr(residual), addr(gelu_src), a_scale_inv.data_ptr(),
+            b_scale_inv.data_ptr(), addr(amax_out), addr(out8), out8_scale.data_ptr() if has8 else None, addr(out8_scale_inv_out) if has8 else None,
+            a.stride(0), b.stride(0), N if out is None else out.stride(0), 0 if residual is None else residual.stride(0),
+            0 if gelu_src is None else gelu_src.stride(0), out8.stride(0) if has8 else 0,
+            M, N, K, native.fmt(a_qtype), native.fmt(b_qtype), native.fmt(out8_qtype) if has8 else 0, int(bool(a_mn)), int(bool(b_mn)),
+            native.dt(out_dtype), 0 if bias is None else native.dt(bias.dtype), 1 if act == 'gelu' else 0, int(max_ctas),
+            int(tile) or _DEFAULT_TILE, addr(stats), addr(colsum_out)
+        )
         native.check(native.lib().msamp_gemm_fp8_ex(ctypes.byref(g), native.stream()), 'gemm_fp8')
         return out
     af = a.view(torch.uint8).view(_F8[a_qtype]).float()

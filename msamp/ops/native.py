@@ -27,6 +27,21 @@ _ERRORS = {
 }
 
 
+# Argument types of the entry points that a layer's forward and backward call: pointers and sizes then go in as plain ints
+# (None = NULL), without a ctypes object per argument.
+_P, _I, _L, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_float
+_ARGTYPES = {
+    'msamp_amax': [_P, _L, _I, _P, _P, _P, _F, _I, _F, _P, _P],
+    'msamp_cast_to_fp8_ex': [_P, _L, _I, _P, _I, _P, _P, _P, _P, _F, _I, _I, _P],
+    'msamp_cast_to_fp8_colsum': [_P, _I, _I, _I, _P, _I, _P, _P, _P, _P, _P, _P],
+    'msamp_layernorm_fwd_q': [_P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _F, _P, _P, _P, _P, _P, _P],
+    'msamp_attention_fwd': [_P] * 6 + [_I] * 4 + [_F, _I, _P],
+    'msamp_attention_tc_fwd': [_P] * 6 + [_I] * 4 + [_F, _I, _P],
+    'msamp_attention_bwd': [_P] * 11 + [_I] * 4 + [_F, _I, _P],
+    'msamp_attention_tc_bwd': [_P] * 11 + [_I] * 4 + [_F, _I, _P],
+}
+
+
 class NativeError(RuntimeError):
     """A native entry point returned a non-zero status."""
 
@@ -62,6 +77,8 @@ def lib():
                     )
                 handle = ctypes.CDLL(LIB_PATH)
                 handle.msamp_last_error.restype = ctypes.c_char_p
+                for name, types in _ARGTYPES.items():
+                    getattr(handle, name).argtypes = types
                 _lib = handle
     return _lib
 
@@ -87,6 +104,18 @@ def stream():
     if _raw_stream is not None and _raw_device is not None:
         return ctypes.c_void_p(_raw_stream(_raw_device()))
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def raw_stream():
+    """The same handle as a plain int, for entry points with declared argument types."""
+    if _raw_stream is not None and _raw_device is not None:
+        return _raw_stream(_raw_device())
+    return torch.cuda.current_stream().cuda_stream
+
+
+def addr(t):
+    """Device address of a tensor as a plain int (None → None)."""
+    return None if t is None else t.data_ptr()
 
 
 def ptr(t):

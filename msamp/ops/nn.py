@@ -85,9 +85,9 @@ def layer_norm_fwd_raw(x2, weight, bias, eps, want_y=True, y8_scale=None, amax_i
         rstd = torch.empty(rows, dtype=torch.float32, device=x2.device)
         native.check(
             native.lib().msamp_layernorm_fwd_q(
-                native.ptr(x2), native.ptr(weight), native.ptr(bias), native.dt(x2.dtype), native.dt(weight.dtype), native.ptr(y),
-                native.ptr(mean), native.ptr(rstd), rows, cols, ctypes.c_float(eps), native.ptr(y8), native.ptr(y8_scale),
-                native.ptr(amax_in), native.ptr(amax_out), native.ptr(scale_inv_out), native.stream()
+                x2.data_ptr(), weight.data_ptr(), native.addr(bias), native.dt(x2.dtype), native.dt(weight.dtype), native.addr(y),
+                mean.data_ptr(), rstd.data_ptr(), rows, cols, eps, native.addr(y8), native.addr(y8_scale), native.addr(amax_in),
+                native.addr(amax_out), native.addr(scale_inv_out), native.raw_stream()
             ), 'layernorm_fwd'
         )
         return y, y8, mean, rstd
@@ -245,6 +245,47 @@ class _AttentionFn(torch.autograd.Function):
         return dq, dk, dv, None, None, None
 
 
+def _packed_strides(B, S, nh, d):
+    """(batch, seq, head) strides of q, k and v inside a contiguous ``[B, S, 3, nh, d]`` tensor, then of a contiguous output."""
+    return [3 * S * nh * d, 3 * nh * d, d] * 3 + [S * nh * d, nh * d, d]
+
+
+def _packed_fwd(qkv, causal, scale):
+    """Attention on a contiguous packed tensor (the callers have checked that): q, k and v are addresses inside it."""
+    B, S, _, nh, d = qkv.shape
+    o = torch.empty((B, S, nh, d), dtype=qkv.dtype, device=qkv.device)
+    lse = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
+    q, sub = qkv.data_ptr(), nh * d * qkv.element_size()
+    native.check(
+        _attn_entry('fwd')(
+            q, q + sub, q + 2 * sub, o.data_ptr(), lse.data_ptr(), _i64x24(*_packed_strides(B, S, nh, d)), B, nh, S, d, scale, int(causal),
+            native.raw_stream()
+        ), 'attention_fwd'
+    )
+    return o, lse
+
+
+def _packed_bwd(qkv, o, lse, d_o, causal, scale):
+    B, S, _, nh, d = qkv.shape
+    if not qkv.is_contiguous():    # a saved tensor may come back with other strides (saved-tensor hooks)
+        qkv = qkv.contiguous()
+    sdo = d_o.stride()
+    if sdo[3] != 1 or any(s % 8 for s in sdo[:3]):
+        d_o = d_o.contiguous()
+        sdo = d_o.stride()
+    dqkv = torch.empty_like(qkv)
+    delta = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
+    packed = _packed_strides(B, S, nh, d)[:9]
+    q, dq, sub = qkv.data_ptr(), dqkv.data_ptr(), nh * d * qkv.element_size()
+    native.check(
+        _attn_entry('bwd')(
+            q, q + sub, q + 2 * sub, o.data_ptr(), lse.data_ptr(), d_o.data_ptr(), dq, dq + sub, dq + 2 * sub, delta.data_ptr(),
+            _i64x24(*packed, *_strides(o), *sdo[:3], *packed), B, nh, S, d, scale, int(causal), native.raw_stream()
+        ), 'attention_bwd'
+    )
+    return dqkv
+
+
 class _AttentionPackedFn(torch.autograd.Function):
     """Attention on a fused ``[B, S, 3, heads, d]`` QKV tensor; the gradient comes back in the same packed layout.
 
@@ -253,17 +294,7 @@ class _AttentionPackedFn(torch.autograd.Function):
     """
     @staticmethod
     def forward(ctx, qkv, causal, scale):
-        B, S, _, nh, d = qkv.shape
-        q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
-        o = torch.empty((B, S, nh, d), dtype=qkv.dtype, device=qkv.device)
-        lse = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
-        st = _strides(q) + _strides(k) + _strides(v) + _strides(o) + [0] * 12
-        native.check(
-            _attn_entry('fwd')(
-                native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(o), native.ptr(lse), _i64x24(*st), B, nh, S, d,
-                ctypes.c_float(scale), int(causal), native.stream()
-            ), 'attention_fwd'
-        )
+        o, lse = _packed_fwd(qkv, causal, scale)
         ctx.save_for_backward(qkv, o, lse)
         ctx.causal, ctx.scale = causal, scale
         return o
@@ -271,22 +302,7 @@ class _AttentionPackedFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, d_o):
         qkv, o, lse = ctx.saved_tensors
-        B, S, _, nh, d = qkv.shape
-        q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
-        if d_o.stride(3) != 1 or any(s % 8 for s in d_o.stride()[:3]):
-            d_o = d_o.contiguous()
-        dqkv = torch.empty_like(qkv)
-        dq, dk, dv = dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]
-        delta = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
-        st = _strides(q) + _strides(k) + _strides(v) + _strides(o) + _strides(d_o) + _strides(dq) + _strides(dk) + _strides(dv)
-        native.check(
-            _attn_entry('bwd')(
-                native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(o), native.ptr(lse), native.ptr(d_o), native.ptr(dq),
-                native.ptr(dk), native.ptr(dv), native.ptr(delta), _i64x24(*st), B, nh, S, d, ctypes.c_float(ctx.scale), int(ctx.causal),
-                native.stream()
-            ), 'attention_bwd'
-        )
-        return dqkv, None, None
+        return _packed_bwd(qkv, o, lse, d_o, ctx.causal, ctx.scale), None, None
 
 
 def attention_qkv_fwd_raw(qkv, causal=True, scale=None):
@@ -296,17 +312,7 @@ def attention_qkv_fwd_raw(qkv, causal=True, scale=None):
     if _use_native(qkv):
         if qkv.dtype != torch.bfloat16 or d not in (64, 128) or not qkv.is_contiguous() or qkv.data_ptr() % 16:
             raise RuntimeError(f'attention_qkv: CUDA kernel needs contiguous bf16 with head_dim 64/128 (got {qkv.dtype}, {d})')
-        q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
-        o = torch.empty((B, S, nh, d), dtype=qkv.dtype, device=qkv.device)
-        lse = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
-        st = _strides(q) + _strides(k) + _strides(v) + _strides(o) + [0] * 12
-        native.check(
-            _attn_entry('fwd')(
-                native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(o), native.ptr(lse), _i64x24(*st), B, nh, S, d,
-                ctypes.c_float(scale), int(causal), native.stream()
-            ), 'attention_fwd'
-        )
-        return o, lse
+        return _packed_fwd(qkv, causal, scale)
     with torch.no_grad():
         return attention(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], causal=causal, scale=scale), None
 
@@ -316,21 +322,7 @@ def attention_qkv_bwd_raw(qkv, o, lse, d_o, causal=True, scale=None):
     B, S, _, nh, d = qkv.shape
     scale = 1.0 / math.sqrt(d) if scale is None else scale
     if _use_native(qkv):
-        q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
-        if d_o.stride(3) != 1 or any(s % 8 for s in d_o.stride()[:3]):
-            d_o = d_o.contiguous()
-        dqkv = torch.empty_like(qkv)
-        dq, dk, dv = dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]
-        delta = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
-        st = _strides(q) + _strides(k) + _strides(v) + _strides(o) + _strides(d_o) + _strides(dq) + _strides(dk) + _strides(dv)
-        native.check(
-            _attn_entry('bwd')(
-                native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(o), native.ptr(lse), native.ptr(d_o), native.ptr(dq),
-                native.ptr(dk), native.ptr(dv), native.ptr(delta), _i64x24(*st), B, nh, S, d, ctypes.c_float(scale), int(causal),
-                native.stream()
-            ), 'attention_bwd'
-        )
-        return dqkv
+        return _packed_bwd(qkv, o, lse, d_o, causal, scale)
     with torch.enable_grad():
         leaf = qkv.detach().clone().requires_grad_(True)
         out = attention(leaf[:, :, 0], leaf[:, :, 1], leaf[:, :, 2], causal=causal, scale=scale)
