@@ -405,6 +405,41 @@ def test_layernorm(dt, shape):
     assert (b.grad - br.grad).abs().max().item() <= tol * math.sqrt(shape[0]) * 2
 
 
+@pytest.mark.parametrize('dt', [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize('rows', [1183, 1184, 5001])    # around the row count from which one warp takes a row (8 per SM)
+@pytest.mark.parametrize('vecs', [1, 31, 33, 95, 129, 257, 511, 512])    # 16-byte vectors per row: edges of the vectors per lane
+def test_layernorm_forward_rows_per_warp(dt, rows, vecs):
+    torch.manual_seed(0)
+    cols = vecs * (4 if dt == torch.float32 else 8)
+    x = (torch.randn(rows, cols, device=DEV) * 2 + 0.5).to(dt)
+    for pdt in (torch.float32, dt):
+        w, b = (torch.rand(cols, device=DEV) + 0.5).to(pdt), torch.randn(cols, device=DEV).to(pdt)
+        am = torch.zeros((), device=DEV)
+        y, _, mean, rstd = K.layer_norm_fwd_raw(x, w, b, 1e-5, amax_out=am)
+        xd = x.double()
+        mu, rs = xd.mean(1), torch.rsqrt(xd.var(1, unbiased=False) + 1e-5)
+        ref = (xd - mu[:, None]) * rs[:, None] * w.double() + b.double()
+        # one rounding to dt (half a unit in the last place: 2^-8 with the 8 significant bits of bf16, 2^-11, 2^-24), and fp32
+        # sums of `cols` terms of size one
+        eps = {torch.bfloat16: 2**-8, torch.float16: 2**-11, torch.float32: 2**-24}[dt]
+        assert ((y.double() - ref).abs() <= eps * ref.abs() * 1.01 + 64 * 2**-24 * rs[:, None] * (xd.abs().amax(1, keepdim=True) + 1)).all()
+        assert am.item() == y.float().abs().max().item()
+
+
+@pytest.mark.parametrize('n', [1, 7, 8 * 256 * 8 + 3, 148 * 6 * 256 * 64 + 8])
+@pytest.mark.parametrize('dt', [torch.bfloat16, torch.float16, torch.float32])
+def test_amax_values(dt, n):
+    """The packed integer maximum: negative zero, the lowest value, infinities and NaN of either sign, anywhere."""
+    x = torch.full((n, ), -0.0, device=DEV, dtype=dt)
+    assert cast.amax(x).item() == 0
+    for v in (-1e-7, 3.0, torch.finfo(dt).min, -float('inf'), float('nan'), -float('nan')):
+        for at in {0, n // 2, n - 1}:
+            y = x.clone()
+            y[at] = v
+            want = float('inf') if v != v else y[at].float().abs().item()
+            assert cast.amax(y).item() == want, (v, at)
+
+
 @pytest.mark.parametrize('shape', [(64, 1024), (300, 4096), (17, 8192), (2500, 4096), (1500, 2048)])
 def test_layernorm_quantised_output_and_residual_backward(shape):
     """LayerNorm that emits e4m3 directly == LayerNorm followed by the cast, bit for bit; backward with the skip gradient."""
