@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kThreads) cast_to_fp8_kernel(const T* __restri
       Bytes16 v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (i + u * stride < nv) v[u] = ld_stream16(xv + i + u * stride);
+        if (i + u * stride < nv) v[u] = xv[i + u * stride];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         if (i + u * stride < nv) {
@@ -315,10 +315,10 @@ __global__ void __launch_bounds__(kThreads) cast_transpose_kernel(const T* __res
         const T* src = x + (int64_t)(r0 + r) * cols + c0 + cc;
         T e[8];
         if constexpr (sizeof(T) == 2) {
-          *reinterpret_cast<Bytes16*>(e) = ld_stream16(src);
+          *reinterpret_cast<Bytes16*>(e) = *reinterpret_cast<const Bytes16*>(src);
         } else {
-          *reinterpret_cast<Bytes16*>(e) = ld_stream16(src);
-          *reinterpret_cast<Bytes16*>(e + 4) = ld_stream16(src + 4);
+          *reinterpret_cast<Bytes16*>(e) = *reinterpret_cast<const Bytes16*>(src);
+          *reinterpret_cast<Bytes16*>(e + 4) = *reinterpret_cast<const Bytes16*>(src + 4);
         }
         uint16_t q[4];
 #pragma unroll

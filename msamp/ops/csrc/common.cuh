@@ -208,21 +208,12 @@ static inline int msamp_grid_for(int64_t work_items, int threads, int ctas_per_s
 struct alignas(16) Bytes16 { uint32_t w[4]; };
 struct alignas(8) Bytes8 { uint32_t w[2]; };
 
-// Streaming loads: data that a kernel reads once is not allocated in L1.  A pure read of 412 MB ran at 5.0 TB/s with plain
-// 16-byte loads, whatever their number in flight, their order or their width, and at 5.9 to 6.0 TB/s with these.
-// ld_stream*: data that no thread writes while the kernel runs.  ld_stream*_rw: data that this thread may store to afterwards.
+// Streaming load of data that no thread writes while the kernel runs: not allocated in L1.  A pure read of 412 MB ran at 5.0 TB/s
+// with plain 16-byte loads, whatever their number in flight, their order or their width, and at 5.9 to 6.0 TB/s with these.
+// For reads only: passes that store about as much as they read, or whose data the next pass wants in L2, were up to 20 % slower
+// with them (FP8 casts, cross-entropy, both passes of add_to_fp8, stage 2 of Adam).
 __device__ __forceinline__ Bytes16 ld_stream16(const void* p) {
   Bytes16 r;
   asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]) : "l"(p));
-  return r;
-}
-__device__ __forceinline__ Bytes16 ld_stream16_rw(const void* p) {
-  Bytes16 r;
-  asm volatile("ld.global.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]) : "l"(p));
-  return r;
-}
-__device__ __forceinline__ Bytes8 ld_stream8_rw(const void* p) {
-  Bytes8 r;
-  asm volatile("ld.global.L1::no_allocate.v2.b32 {%0, %1}, [%2];" : "=r"(r.w[0]), "=r"(r.w[1]) : "l"(p));
   return r;
 }
