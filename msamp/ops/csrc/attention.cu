@@ -614,6 +614,7 @@ MSAMP_API int msamp_attention_fwd(const void* q, const void* k, const void* v, v
                                   int heads, int seqlen, int head_dim, float scale, int causal, void* stream_) {
   MSAMP_REQUIRE(head_dim == 64 || head_dim == 128, "attention: head_dim must be 64 or 128 (got %d)", head_dim);
   MSAMP_REQUIRE(batch > 0 && heads > 0 && seqlen > 0, "attention: empty problem");
+  MSAMP_REQUIRE(aligned16(q) && aligned16(k) && aligned16(v) && aligned16(o), "attention: q, k, v and o must be 16-byte aligned");
   for (int i = 0; i < 12; ++i) MSAMP_REQUIRE(strides[i] % 8 == 0, "attention: stride %d is not a multiple of 8 elements", i);
   AttnParams p = {};
   p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v; p.o = (__nv_bfloat16*)o; p.lse = lse;
@@ -631,6 +632,8 @@ MSAMP_API int msamp_attention_bwd(const void* q, const void* k, const void* v, c
                                   int head_dim, float scale, int causal, void* stream_) {
   MSAMP_REQUIRE(head_dim == 64 || head_dim == 128, "attention: head_dim must be 64 or 128 (got %d)", head_dim);
   MSAMP_REQUIRE(batch > 0 && heads > 0 && seqlen > 0, "attention: empty problem");
+  MSAMP_REQUIRE(aligned16(q) && aligned16(k) && aligned16(v) && aligned16(o) && aligned16(d_o) && aligned16(dq) && aligned16(dk) && aligned16(dv),
+                "attention: q, k, v, o, dO and the gradients must be 16-byte aligned");
   for (int i = 0; i < 24; ++i) MSAMP_REQUIRE(strides[i] % 8 == 0, "attention: stride %d is not a multiple of 8 elements", i);
   AttnParams p = {};
   p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v; p.o = (__nv_bfloat16*)const_cast<void*>(o);

@@ -3043,53 +3043,53 @@ extern "C" int msamp_attention_bwd(const void*, const void*, const void*, const 
 
 // Same contract as msamp_attention_fwd (attention.cu), head_dim 64 or 128: strides are the (batch, seq, head)
 // element strides of q, k, v, o; every pointer 16-byte aligned, every stride a multiple of 8 elements.
+// All checks and tensor maps come before the first launch, so that a call that is refused has queued nothing.
 MSAMP_API int msamp_attention_tc_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int64_t* strides, int batch,
                                      int heads, int seqlen, int head_dim, float scale, int causal, void* stream_) {
   MSAMP_REQUIRE(head_dim == 64 || head_dim == 128, "attention (tcgen05): head_dim must be 64 or 128 (got %d)", head_dim);
   MSAMP_REQUIRE(batch > 0 && heads > 0 && seqlen > 0, "attention: empty problem");
+  MSAMP_REQUIRE(aligned16(q) && aligned16(k) && aligned16(v) && aligned16(o), "attention: q, k, v and o must be 16-byte aligned");
   for (int i = 0; i < 12; ++i) MSAMP_REQUIRE(strides[i] % 8 == 0, "attention: stride %d is not a multiple of 8 elements", i);
   if (has_repeats(strides, 3, batch, heads, seqlen))
     return msamp_attention_fwd(q, k, v, o, lse, strides, batch, heads, seqlen, head_dim, scale, causal, stream_);
+  // MSAMP_ATTN_FWD_SMEM=1 selects the kernel with 64-key score tiles and P in shared memory (default: 128-key score
+  // tiles, P in tensor memory), MSAMP_ATTN_FWD_PERSIST=0 one CTA per (query tile, batch, head) instead of persistent CTAs.
+  static const bool smem_env = [] { const char* e = getenv("MSAMP_ATTN_FWD_SMEM"); return e && e[0] == '1'; }();
+  static const bool persist_env = [] { const char* e = getenv("MSAMP_ATTN_FWD_PERSIST"); return !(e && e[0] == '0'); }();
+  const bool smem_operands = smem_env && head_dim == 128, persistent = persist_env || head_dim == 64;
+  const int k_rows = smem_operands ? 64 : 128, v_rows = !smem_operands && persistent ? 128 : 64;
   CUtensorMap mq, mk, mv;
   int rc;
   if ((rc = make_map4(q, batch, heads, seqlen, head_dim, strides[0], strides[1], strides[2], 128, &mq))) return rc;
-  if ((rc = make_map4(k, batch, heads, seqlen, head_dim, strides[3], strides[4], strides[5], 64, &mk))) return rc;
-  if ((rc = make_map4(v, batch, heads, seqlen, head_dim, strides[6], strides[7], strides[8], 64, &mv))) return rc;
+  if ((rc = make_map4(k, batch, heads, seqlen, head_dim, strides[3], strides[4], strides[5], k_rows, &mk))) return rc;
+  if ((rc = make_map4(v, batch, heads, seqlen, head_dim, strides[6], strides[7], strides[8], v_rows, &mv))) return rc;
   TcParams p = {};
   p.o = (__nv_bfloat16*)o; p.lse = lse;
   p.o_sb = strides[9]; p.o_ss = strides[10]; p.o_sh = strides[11];
   p.batch = batch; p.heads = heads; p.seqlen = seqlen; p.causal = causal; p.scale = scale;
   p.status = msamp_device_status_ptr();
   p.group = item_group(seqlen, head_dim);
-  dim3 grid((seqlen + 127) / 128, batch * heads);
-  // MSAMP_ATTN_FWD_SMEM=1 selects the kernel with 64-key score tiles and P in shared memory (default: 128-key score
-  // tiles, P in tensor memory).
-  static const bool smem_operands = [] { const char* e = getenv("MSAMP_ATTN_FWD_SMEM"); return e && e[0] == '1'; }();
-  if (smem_operands && head_dim == 128) {
+  cudaStream_t stream = (cudaStream_t)stream_;
+  const int n_qt = (seqlen + 127) / 128;
+  dim3 grid(n_qt, batch * heads);
+  if (smem_operands) {
     if ((rc = set_smem(attn_fwd_tc_kernel, fwd::SMEM))) return rc;
-    attn_fwd_tc_kernel<<<grid, kTcThreads, fwd::SMEM, (cudaStream_t)stream_>>>(mq, mk, mv, p);
+    attn_fwd_tc_kernel<<<grid, kTcThreads, fwd::SMEM, stream>>>(mq, mk, mv, p);
     return msamp_check_launch("attn_fwd_tc_kernel");
   }
-  CUtensorMap mk128;
-  if ((rc = make_map4(k, batch, heads, seqlen, head_dim, strides[3], strides[4], strides[5], 128, &mk128))) return rc;
-  // MSAMP_ATTN_FWD_PERSIST=0 launches one CTA per (query tile, batch, head) instead of persistent CTAs
-  static const bool persistent = [] { const char* e = getenv("MSAMP_ATTN_FWD_PERSIST"); return !(e && e[0] == '0'); }();
-  if (!persistent && head_dim == 128) {
+  if (!persistent) {
     if ((rc = set_smem(attn_fwd_tm_kernel, fwd2::SMEM))) return rc;
-    attn_fwd_tm_kernel<<<grid, kTcThreads, fwd2::SMEM, (cudaStream_t)stream_>>>(mq, mk128, mv, p);
+    attn_fwd_tm_kernel<<<grid, kTcThreads, fwd2::SMEM, stream>>>(mq, mk, mv, p);
     return msamp_check_launch("attn_fwd_tm_kernel");
   }
-  const int n_qt = (seqlen + 127) / 128;
   const int n_items = n_qt * batch * heads;
   const int ctas = n_items < msamp_sm_count() ? n_items : msamp_sm_count();
-  CUtensorMap mv128;
-  if ((rc = make_map4(v, batch, heads, seqlen, head_dim, strides[6], strides[7], strides[8], 128, &mv128))) return rc;
   if (head_dim == 128) {
     if ((rc = set_smem(attn_fwd_ps_kernel<128>, fwd3::Cfg<128>::SMEM))) return rc;
-    attn_fwd_ps_kernel<128><<<ctas, kPsThreads, fwd3::Cfg<128>::SMEM, (cudaStream_t)stream_>>>(mq, mk128, mv128, p, n_qt, n_items);
+    attn_fwd_ps_kernel<128><<<ctas, kPsThreads, fwd3::Cfg<128>::SMEM, stream>>>(mq, mk, mv, p, n_qt, n_items);
   } else {
     if ((rc = set_smem(attn_fwd_ps_kernel<64>, fwd3::Cfg<64>::SMEM))) return rc;
-    attn_fwd_ps_kernel<64><<<ctas, kPsThreads, fwd3::Cfg<64>::SMEM, (cudaStream_t)stream_>>>(mq, mk128, mv128, p, n_qt, n_items);
+    attn_fwd_ps_kernel<64><<<ctas, kPsThreads, fwd3::Cfg<64>::SMEM, stream>>>(mq, mk, mv, p, n_qt, n_items);
   }
   return msamp_check_launch("attn_fwd_ps_kernel");
 }
@@ -3100,9 +3100,29 @@ MSAMP_API int msamp_attention_tc_bwd(const void* q, const void* k, const void* v
                                      int seqlen, int head_dim, float scale, int causal, void* stream_) {
   MSAMP_REQUIRE(head_dim == 64 || head_dim == 128, "attention (tcgen05): head_dim must be 64 or 128 (got %d)", head_dim);
   MSAMP_REQUIRE(batch > 0 && heads > 0 && seqlen > 0, "attention: empty problem");
+  MSAMP_REQUIRE(aligned16(q) && aligned16(k) && aligned16(v) && aligned16(o) && aligned16(d_o) && aligned16(dq) && aligned16(dk) && aligned16(dv),
+                "attention: q, k, v, o, dO and the gradients must be 16-byte aligned");
   for (int i = 0; i < 24; ++i) MSAMP_REQUIRE(strides[i] % 8 == 0, "attention: stride %d is not a multiple of 8 elements", i);
   if (has_repeats(strides, 5, batch, heads, seqlen))
     return msamp_attention_bwd(q, k, v, o, lse, d_o, dq, dk, dv, delta, strides, batch, heads, seqlen, head_dim, scale, causal, stream_);
+  // MSAMP_ATTN_BWD_SMEM=1 selects the kernels with 64-wide score tiles and the second operand in shared memory,
+  // MSAMP_ATTN_BWD_PERSIST=0 one CTA per (tile, batch, head) instead of persistent CTAs over the work items
+  static const bool smem_env = [] { const char* e = getenv("MSAMP_ATTN_BWD_SMEM"); return e && e[0] == '1'; }();
+  static const bool persist_env = [] { const char* e = getenv("MSAMP_ATTN_BWD_PERSIST"); return !(e && e[0] == '0'); }();
+  const bool smem_operands = smem_env && head_dim == 128, persistent = persist_env || head_dim == 64;
+  // boxes of 128 rows throughout, except for the operand that the 64-wide kernels stream
+  CUtensorMap mq, mk, mv, mdo, mq64, mk64, mv64, mdo64;
+  int rc;
+  if ((rc = make_map4(q, batch, heads, seqlen, head_dim, strides[0], strides[1], strides[2], 128, &mq))) return rc;
+  if ((rc = make_map4(k, batch, heads, seqlen, head_dim, strides[3], strides[4], strides[5], 128, &mk))) return rc;
+  if ((rc = make_map4(v, batch, heads, seqlen, head_dim, strides[6], strides[7], strides[8], 128, &mv))) return rc;
+  if ((rc = make_map4(d_o, batch, heads, seqlen, head_dim, strides[12], strides[13], strides[14], 128, &mdo))) return rc;
+  if (smem_operands) {
+    if ((rc = make_map4(q, batch, heads, seqlen, head_dim, strides[0], strides[1], strides[2], 64, &mq64))) return rc;
+    if ((rc = make_map4(k, batch, heads, seqlen, head_dim, strides[3], strides[4], strides[5], 64, &mk64))) return rc;
+    if ((rc = make_map4(v, batch, heads, seqlen, head_dim, strides[6], strides[7], strides[8], 64, &mv64))) return rc;
+    if ((rc = make_map4(d_o, batch, heads, seqlen, head_dim, strides[12], strides[13], strides[14], 64, &mdo64))) return rc;
+  }
   cudaStream_t stream = (cudaStream_t)stream_;
   {
     DeltaParams d = {};
@@ -3125,74 +3145,30 @@ MSAMP_API int msamp_attention_tc_bwd(const void* q, const void* k, const void* v
   p.batch = batch; p.heads = heads; p.seqlen = seqlen; p.causal = causal; p.scale = scale;
   p.status = msamp_device_status_ptr();
   p.group = item_group(seqlen, head_dim);
-  int rc;
-  {
-    CUtensorMap mq, mk, mv, mdo;
-    if ((rc = make_map4(q, batch, heads, seqlen, head_dim, strides[0], strides[1], strides[2], 64, &mq))) return rc;
-    if ((rc = make_map4(k, batch, heads, seqlen, head_dim, strides[3], strides[4], strides[5], 128, &mk))) return rc;
-    if ((rc = make_map4(v, batch, heads, seqlen, head_dim, strides[6], strides[7], strides[8], 128, &mv))) return rc;
-    if ((rc = make_map4(d_o, batch, heads, seqlen, head_dim, strides[12], strides[13], strides[14], 64, &mdo))) return rc;
-    dim3 grid((seqlen + 127) / 128, batch * heads);
-    static const bool smem_operands = [] { const char* e = getenv("MSAMP_ATTN_BWD_SMEM"); return e && e[0] == '1'; }();
-    if (smem_operands && head_dim == 128) {
-      if ((rc = set_smem(attn_bwd_dkdv_tc_kernel, dkv::SMEM))) return rc;
-      attn_bwd_dkdv_tc_kernel<<<grid, kTcThreads, dkv::SMEM, stream>>>(mq, mk, mv, mdo, p);
-    } else {
-      CUtensorMap mq128, mdo128;
-      if ((rc = make_map4(q, batch, heads, seqlen, head_dim, strides[0], strides[1], strides[2], 128, &mq128))) return rc;
-      if ((rc = make_map4(d_o, batch, heads, seqlen, head_dim, strides[12], strides[13], strides[14], 128, &mdo128))) return rc;
-      static const bool persistent = [] { const char* e = getenv("MSAMP_ATTN_BWD_PERSIST"); return !(e && e[0] == '0'); }();
-      if (persistent || head_dim == 64) {
-        const int n_kt = (seqlen + 127) / 128;
-        const int n_items = n_kt * batch * heads;
-        const int ctas = n_items < msamp_sm_count() ? n_items : msamp_sm_count();
-        if (head_dim == 128) {
-          if ((rc = set_smem(attn_bwd_dkdv_ps_kernel<128>, dkv3::Cfg<128>::SMEM))) return rc;
-          attn_bwd_dkdv_ps_kernel<128><<<ctas, kPsThreads, dkv3::Cfg<128>::SMEM, stream>>>(mq128, mk, mv, mdo128, p, n_kt, n_items);
-        } else {
-          if ((rc = set_smem(attn_bwd_dkdv_ps_kernel<64>, dkv3::Cfg<64>::SMEM))) return rc;
-          attn_bwd_dkdv_ps_kernel<64><<<ctas, kPsThreads, dkv3::Cfg<64>::SMEM, stream>>>(mq128, mk, mv, mdo128, p, n_kt, n_items);
-        }
-      } else {
-        if ((rc = set_smem(attn_bwd_dkdv_tm_kernel, dkv2::SMEM))) return rc;
-        attn_bwd_dkdv_tm_kernel<<<grid, kTcThreads, dkv2::SMEM, stream>>>(mq128, mk, mv, mdo128, p);
-      }
-    }
-  }
-  {
-    CUtensorMap mq, mk, mv, mdo;
-    if ((rc = make_map4(q, batch, heads, seqlen, head_dim, strides[0], strides[1], strides[2], 128, &mq))) return rc;
-    if ((rc = make_map4(k, batch, heads, seqlen, head_dim, strides[3], strides[4], strides[5], 64, &mk))) return rc;
-    if ((rc = make_map4(v, batch, heads, seqlen, head_dim, strides[6], strides[7], strides[8], 64, &mv))) return rc;
-    if ((rc = make_map4(d_o, batch, heads, seqlen, head_dim, strides[12], strides[13], strides[14], 128, &mdo))) return rc;
-    dim3 grid((seqlen + 127) / 128, batch * heads);
-    // MSAMP_ATTN_BWD_SMEM=1 selects the kernels with 64-wide score tiles and the second operand in shared memory
-    static const bool smem_operands = [] { const char* e = getenv("MSAMP_ATTN_BWD_SMEM"); return e && e[0] == '1'; }();
-    if (smem_operands && head_dim == 128) {
-      if ((rc = set_smem(attn_bwd_dq_tc_kernel, dqk::SMEM))) return rc;
-      attn_bwd_dq_tc_kernel<<<grid, kTcThreads, dqk::SMEM, stream>>>(mq, mk, mv, mdo, p);
-    } else {
-      CUtensorMap mk128, mv128;
-      if ((rc = make_map4(k, batch, heads, seqlen, head_dim, strides[3], strides[4], strides[5], 128, &mk128))) return rc;
-      if ((rc = make_map4(v, batch, heads, seqlen, head_dim, strides[6], strides[7], strides[8], 128, &mv128))) return rc;
-      // MSAMP_ATTN_BWD_PERSIST=0: one CTA per (tile, batch, head) instead of persistent CTAs over the work items
-      static const bool persistent = [] { const char* e = getenv("MSAMP_ATTN_BWD_PERSIST"); return !(e && e[0] == '0'); }();
-      if (persistent || head_dim == 64) {
-        const int n_qt = (seqlen + 127) / 128;
-        const int n_items = n_qt * batch * heads;
-        const int ctas = n_items < msamp_sm_count() ? n_items : msamp_sm_count();
-        if (head_dim == 128) {
-          if ((rc = set_smem(attn_bwd_dq_ps_kernel<128>, dqk3::Cfg<128>::SMEM))) return rc;
-          attn_bwd_dq_ps_kernel<128><<<ctas, kPsThreads, dqk3::Cfg<128>::SMEM, stream>>>(mq, mk128, mv128, mdo, p, n_qt, n_items);
-        } else {
-          if ((rc = set_smem(attn_bwd_dq_ps_kernel<64>, dqk3::Cfg<64>::SMEM))) return rc;
-          attn_bwd_dq_ps_kernel<64><<<ctas, kPsThreads, dqk3::Cfg<64>::SMEM, stream>>>(mq, mk128, mv128, mdo, p, n_qt, n_items);
-        }
-      } else {
-        if ((rc = set_smem(attn_bwd_dq_tm_kernel, dqk2::SMEM))) return rc;
-        attn_bwd_dq_tm_kernel<<<grid, kTcThreads, dqk2::SMEM, stream>>>(mq, mk128, mv128, mdo, p);
-      }
-    }
+  const int n_t = (seqlen + 127) / 128;    // key tiles of dK / dV, query tiles of dQ
+  const int n_items = n_t * batch * heads;
+  const int ctas = n_items < msamp_sm_count() ? n_items : msamp_sm_count();
+  dim3 grid(n_t, batch * heads);
+  if (smem_operands) {
+    if ((rc = set_smem(attn_bwd_dkdv_tc_kernel, dkv::SMEM))) return rc;
+    attn_bwd_dkdv_tc_kernel<<<grid, kTcThreads, dkv::SMEM, stream>>>(mq64, mk, mv, mdo64, p);
+    if ((rc = set_smem(attn_bwd_dq_tc_kernel, dqk::SMEM))) return rc;
+    attn_bwd_dq_tc_kernel<<<grid, kTcThreads, dqk::SMEM, stream>>>(mq, mk64, mv64, mdo, p);
+  } else if (!persistent) {
+    if ((rc = set_smem(attn_bwd_dkdv_tm_kernel, dkv2::SMEM))) return rc;
+    attn_bwd_dkdv_tm_kernel<<<grid, kTcThreads, dkv2::SMEM, stream>>>(mq, mk, mv, mdo, p);
+    if ((rc = set_smem(attn_bwd_dq_tm_kernel, dqk2::SMEM))) return rc;
+    attn_bwd_dq_tm_kernel<<<grid, kTcThreads, dqk2::SMEM, stream>>>(mq, mk, mv, mdo, p);
+  } else if (head_dim == 128) {
+    if ((rc = set_smem(attn_bwd_dkdv_ps_kernel<128>, dkv3::Cfg<128>::SMEM))) return rc;
+    attn_bwd_dkdv_ps_kernel<128><<<ctas, kPsThreads, dkv3::Cfg<128>::SMEM, stream>>>(mq, mk, mv, mdo, p, n_t, n_items);
+    if ((rc = set_smem(attn_bwd_dq_ps_kernel<128>, dqk3::Cfg<128>::SMEM))) return rc;
+    attn_bwd_dq_ps_kernel<128><<<ctas, kPsThreads, dqk3::Cfg<128>::SMEM, stream>>>(mq, mk, mv, mdo, p, n_t, n_items);
+  } else {
+    if ((rc = set_smem(attn_bwd_dkdv_ps_kernel<64>, dkv3::Cfg<64>::SMEM))) return rc;
+    attn_bwd_dkdv_ps_kernel<64><<<ctas, kPsThreads, dkv3::Cfg<64>::SMEM, stream>>>(mq, mk, mv, mdo, p, n_t, n_items);
+    if ((rc = set_smem(attn_bwd_dq_ps_kernel<64>, dqk3::Cfg<64>::SMEM))) return rc;
+    attn_bwd_dq_ps_kernel<64><<<ctas, kPsThreads, dqk3::Cfg<64>::SMEM, stream>>>(mq, mk, mv, mdo, p, n_t, n_items);
   }
   return msamp_check_launch("attn_bwd_tc kernels");
 }

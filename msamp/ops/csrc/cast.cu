@@ -481,8 +481,6 @@ __global__ void roll_windows_kernel(float* amax, float* scale, int* bad, int n, 
   if (bad != nullptr) bad[i] = finite ? 0 : 1;
 }
 
-inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-inline bool aligned8(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; }
 
 }    // namespace
 

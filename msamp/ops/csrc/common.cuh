@@ -205,6 +205,9 @@ static inline int msamp_grid_for(int64_t work_items, int threads, int ctas_per_s
   return (int)(need < cap ? need : cap);
 }
 
+static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+static inline bool aligned8(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; }
+
 struct alignas(16) Bytes16 { uint32_t w[4]; };
 struct alignas(8) Bytes8 { uint32_t w[2]; };
 

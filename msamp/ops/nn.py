@@ -203,6 +203,15 @@ def _strides(t):
     return [t.stride(0), t.stride(1), t.stride(2)]
 
 
+def _rows16(t):
+    """``t`` if its rows can be read 16 bytes at a time (unit inner stride, other strides and start in whole 16 bytes), else a
+    contiguous copy: an incoming gradient may be a view with any strides that starts anywhere in its buffer."""
+    s = t.stride()
+    if s[3] != 1 or s[0] % 8 or s[1] % 8 or s[2] % 8 or t.data_ptr() % 16:
+        t = t.clone(memory_format=torch.contiguous_format)
+    return t
+
+
 class _AttentionFn(torch.autograd.Function):
     """Inputs are [B, S, nh, d] bf16 views (arbitrary batch/seq/head strides); output is contiguous [B, S, nh, d]."""
     @staticmethod
@@ -225,8 +234,7 @@ class _AttentionFn(torch.autograd.Function):
     def backward(ctx, d_o):
         q, k, v, o, lse = ctx.saved_tensors
         B, S, nh, d = q.shape
-        if d_o.stride(3) != 1:
-            d_o = d_o.contiguous()
+        o, d_o = _rows16(o), _rows16(d_o)
         if ctx.grad_layout == 'packed':
             # one [B, S, 3, nh, d] buffer so that the gradient of a fused QKV projection needs no concatenation
             dqkv = torch.empty((B, S, 3, nh, d), dtype=q.dtype, device=q.device)
@@ -267,12 +275,9 @@ def _packed_fwd(qkv, causal, scale):
 
 def _packed_bwd(qkv, o, lse, d_o, causal, scale):
     B, S, _, nh, d = qkv.shape
-    if not qkv.is_contiguous():    # a saved tensor may come back with other strides (saved-tensor hooks)
-        qkv = qkv.contiguous()
-    sdo = d_o.stride()
-    if sdo[3] != 1 or any(s % 8 for s in sdo[:3]):
-        d_o = d_o.contiguous()
-        sdo = d_o.stride()
+    if not qkv.is_contiguous() or qkv.data_ptr() % 16:    # a saved tensor may come back with other strides (saved-tensor hooks)
+        qkv = qkv.clone(memory_format=torch.contiguous_format)
+    o, d_o = _rows16(o), _rows16(d_o)
     dqkv = torch.empty_like(qkv)
     delta = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
     packed = _packed_strides(B, S, nh, d)[:9]
@@ -280,7 +285,7 @@ def _packed_bwd(qkv, o, lse, d_o, causal, scale):
     native.check(
         _attn_entry('bwd')(
             q, q + sub, q + 2 * sub, o.data_ptr(), lse.data_ptr(), d_o.data_ptr(), dq, dq + sub, dq + 2 * sub, delta.data_ptr(),
-            _i64x24(*packed, *_strides(o), *sdo[:3], *packed), B, nh, S, d, scale, int(causal), native.raw_stream()
+            _i64x24(*packed, *_strides(o), *_strides(d_o), *packed), B, nh, S, d, scale, int(causal), native.raw_stream()
         ), 'attention_bwd'
     )
     return dqkv

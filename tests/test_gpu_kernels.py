@@ -658,6 +658,25 @@ def test_attention_repeated_heads(d):
         assert _rel(got.grad, ref.grad) <= 3 * 2**-9
 
 
+@pytest.mark.parametrize('d', [64, 128])
+@pytest.mark.parametrize('packed', [True, False])
+def test_attention_output_in_a_concatenation(d, packed):
+    """The backward of a concatenation hands over a gradient that starts 8 bytes into its buffer: it is copied, not read in place."""
+    torch.manual_seed(3)
+    B, S, H = 2, 70, 3
+    qkv = torch.randn(B, S, 3, H, d, device=DEV, dtype=torch.bfloat16).requires_grad_()
+    side = torch.randn(B, S, H, 4, device=DEV, dtype=torch.bfloat16)
+    out = K.attention_qkv(qkv) if packed else K.attention(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2])
+    seen = []
+    out.register_hook(lambda g: seen.append((g.data_ptr() % 16, g.clone(memory_format=torch.contiguous_format))))
+    cat = torch.cat([side, out, side], -1)
+    cat.backward(torch.randn(B, S, H, d + 8, device=DEV, dtype=torch.bfloat16))
+    assert seen[0][0] == 8
+    other = qkv.detach().clone().requires_grad_()
+    K.attention_qkv(other).backward(seen[0][1])
+    assert torch.equal(qkv.grad, other.grad)
+
+
 def test_cross_entropy():
     torch.manual_seed(0)
     rows, vocab = 300, 50304
