@@ -2988,6 +2988,15 @@ int make_map4(const void* ptr, int batch, int heads, int seqlen, int head_dim, i
     msamp_set_error("cuTensorMapEncodeTiled is not available from the driver");
     return MSAMP_ETMAP;
   }
+  // The driver call needs a current context.  A thread whose first CUDA call this is (autograd runs backward in threads of its
+  // own) has none yet; setting the device that it is on makes the primary one current.
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaSetDevice(dev);
+  if (e != cudaSuccess) {
+    msamp_set_error("attention: no CUDA context: %s", cudaGetErrorString(e));
+    return MSAMP_ELAUNCH;
+  }
   // A dimension of extent 1 still needs a valid (16-byte multiple) stride.
   cuuint64_t dims[4] = {(cuuint64_t)head_dim, (cuuint64_t)heads, (cuuint64_t)seqlen, (cuuint64_t)batch};
   cuuint64_t strides[3] = {(cuuint64_t)sh * 2, (cuuint64_t)ss * 2, (cuuint64_t)sb * 2};
