@@ -200,25 +200,25 @@ struct Elem {
   float p, m, v;
 };
 
+// One definition of the update: the order of the operations and which of them are fused are written out, here and in adam_elem2,
+// so that every path (vector loop, tail, unaligned tensors, the reduction inside stage 1) and both stages give the same bits.
 __device__ __forceinline__ Elem adam_elem(const AdamTensor& t, float p, float g, float m, float v, float psi, float gsi, float msi,
                                           float vsi) {
-  p *= psi;
-  g = g * gsi * t.gsign;
-  g += t.l2 * p;
-  p *= t.lr_wd_factor;
+  p = __fmul_rn(p, psi);
+  g = __fmaf_rn(__fmul_rn(g, gsi), t.gsign, __fmul_rn(t.l2, p));
   Elem e;
-  e.m = t.beta1 * (m * msi) + (1.0f - t.beta1) * g;
-  e.v = t.beta2 * (v * vsi) + (1.0f - t.beta2) * (g * g);
+  e.m = __fmaf_rn(t.beta1, __fmul_rn(m, msi), __fmul_rn(1.0f - t.beta1, g));
+  e.v = __fmaf_rn(t.beta2, __fmul_rn(v, vsi), __fmul_rn(1.0f - t.beta2, __fmul_rn(g, g)));
   // sqrt and the division use the hardware approximations (about 1 ulp): the kernel is otherwise bound by
   // instruction issue, not by memory, and Adam is insensitive to errors of that size
   float root;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(root) : "f"(e.v));
-  float denom = root * t.inv_sqrt_bc2 + t.eps;
-  e.p = p - t.step_size * __fdividef(e.m, denom);
+  const float denom = __fmaf_rn(root, t.inv_sqrt_bc2, t.eps);
+  e.p = __fmaf_rn(p, t.lr_wd_factor, __fmul_rn(-t.step_size, __fdividef(e.m, denom)));
   return e;
 }
 
-// Two elements at once (f32x2: the roundings of adam_elem at half the issue slots).
+// Two elements at once: the operations of adam_elem in the same order, as f32x2 at half the issue slots.
 struct Elem2 {
   uint64_t p, m, v;
 };
@@ -233,10 +233,8 @@ struct AdamConst2 {
   }
 };
 __device__ __forceinline__ Elem2 adam_elem2(const AdamConst2& k, float p0, float p1, float g0, float g1, float m0, float m1, float v0, float v1) {
-  uint64_t p = f2_mul(f2_pack(p0, p1), k.psi);
-  uint64_t g = f2_mul(f2_mul(f2_pack(g0, g1), k.gsi), k.gsign);
-  g = f2_fma(k.l2, p, g);
-  p = f2_mul(p, k.wd);
+  const uint64_t p = f2_mul(f2_pack(p0, p1), k.psi);
+  const uint64_t g = f2_fma(f2_mul(f2_pack(g0, g1), k.gsi), k.gsign, f2_mul(k.l2, p));
   Elem2 e;
   e.m = f2_fma(k.b1, f2_mul(f2_pack(m0, m1), k.msi), f2_mul(k.b1c, g));
   e.v = f2_fma(k.b2, f2_mul(f2_pack(v0, v1), k.vsi), f2_mul(k.b2c, f2_mul(g, g)));
@@ -245,7 +243,7 @@ __device__ __forceinline__ Elem2 adam_elem2(const AdamConst2& k, float p0, float
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(v.x));
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(v.y));
   const float2 d = f2_unpack(f2_fma(f2_pack(r0, r1), k.isb, k.eps));
-  e.p = f2_fma(k.nstep, f2_pack(__fdividef(m.x, d.x), __fdividef(m.y, d.y)), p);
+  e.p = f2_fma(p, k.wd, f2_mul(k.nstep, f2_pack(__fdividef(m.x, d.x), __fdividef(m.y, d.y))));
   return e;
 }
 

@@ -382,6 +382,83 @@ def test_fused_adam_matches_definition(p_kind, state_dtypes, use_adam):
         assert (vg - vc).abs().max().item() <= 0.02 * vc.abs().max().item() + 1e-9
 
 
+_ADAM_KINDS = {'f32': torch.float32, 'f16': torch.float16, 'bf16': torch.bfloat16, 'e4m3': E4, 'e5m2': E5, 'scaled16': Dtypes.kfloat16}
+
+
+def _adam_entry(kinds, n, offset, seed):
+    """One descriptor of the fused step with non-zero moments; every tensor starts ``offset`` elements into its buffer."""
+    from msamp.common.tensor import ScalingTensor
+    gen = torch.Generator().manual_seed(seed)
+    e = dict(lr_wd_factor=1 - 1e-3, l2=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, step_size=1e-2, sqrt_bc2=0.8, gsign=1.0, tensor_scale=True)
+    for name, kind, size in zip('pgmv', kinds, (1.0, 1e-2, 1e-2, 1e-4)):
+        x = torch.randn(n, generator=gen) * size
+        x = (x.abs() if name == 'v' else x).to(DEV)
+        kind = _ADAM_KINDS[kind]
+        t = x.cast(kind) if isinstance(kind, type(E4)) else x.to(kind)
+        val = t.value if isinstance(t, ScalingTensor) else t
+        buf = torch.empty(n + offset, dtype=val.dtype, device=DEV)
+        buf[offset:] = val
+        e[name] = ScalingTensor(buf[offset:], t.meta) if isinstance(t, ScalingTensor) else buf[offset:]
+    return e
+
+
+def _adam_result(e):
+    from msamp.common.tensor import ScalingTensor
+    out = []
+    for name in 'pmv':
+        t = e[name]
+        if isinstance(t, ScalingTensor):
+            out += [t.value.cpu(), t.meta.scale.cpu(), t.meta.scale_inv.cpu(), t.meta.amax[0].cpu()]
+        else:
+            out.append(t.cpu())
+    return out
+
+
+# a chunk is 16384 elements, a step of the vector loop 2048: one vector and a tail, the loop's remainder, several chunks
+@pytest.mark.parametrize('n', [13, 2048 * 3 + 8, 16384 * 2 + 2048 * 5 + 13])
+@pytest.mark.parametrize('kinds', [('f32', 'f32', 'f32', 'f32'), ('scaled16', 'e4m3', 'e4m3', 'f16'), ('bf16', 'bf16', 'f32', 'f32'),
+                                   ('f32', 'bf16', 'e5m2', 'f16')])
+def test_fused_adam_same_bits_on_every_path(kinds, n):
+    """Aligned tensors (vector loop, then a tail) and unaligned ones (element by element) give the same bits."""
+    from msamp.ops.optim import FusedPlan
+    plan = FusedPlan(torch.device(DEV, 0))
+    results = []
+    for offset in (0, 1):
+        e = _adam_entry(kinds, n, offset, seed=5)
+        plan.run([e])
+        results.append(_adam_result(e))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
+def test_fused_adam_reduction_of_one_rank_same_bits():
+    """Stage 1 with the gradient reduction folded in, for a group of one rank, against the plain step: the gradient's bytes and scale
+    come back unchanged, so maxima, scales and stored values agree bit for bit."""
+    import ctypes
+    from msamp.ops.optim import FusedPlan
+    plan, sizes = FusedPlan(torch.device(DEV, 0)), [16384 + 2048 * 3 + 5] * 12
+    kinds = ('scaled16', 'e4m3', 'e4m3', 'f16')
+    results = []
+    for fused in (False, True):
+        entries = [_adam_entry(kinds, n, 0, seed=i) for i, n in enumerate(sizes)]
+        reduce_args = None
+        if fused:
+            step = (max(sizes) + 255) // 256 * 256
+            flat = torch.zeros(step * len(sizes), dtype=torch.uint8, device=DEV)
+            meta = torch.zeros(3, len(sizes), device=DEV)
+            for i, e in enumerate(entries):
+                g = e['g']
+                flat[i * step:i * step + sizes[i]] = g.value
+                meta[0, i], meta[1, i] = g.meta.scale_inv, g.meta.amax[0]
+                g.value, e['g_index'] = flat[i * step:i * step + sizes[i]], i
+            reduce_args = dict(data_table=(ctypes.c_void_p * 1)(flat.data_ptr()), meta_table=(ctypes.c_void_p * 1)(meta.data_ptr()), world=1, rank=0,
+                               n_tensors=len(sizes))
+        plan.run(entries, reduce_args)
+        results.append([r for e in entries for r in _adam_result(e)])
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize('dt', [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize('shape', [(64, 256), (1000, 4096), (7, 1024), (3, 8192), (2500, 4096), (1300, 1024)])    # the last two: bulk-copy backward
 def test_layernorm(dt, shape):
