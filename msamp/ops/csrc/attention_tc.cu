@@ -8,6 +8,7 @@
 //   attn_fwd_ps_kernel        forward, 128 queries x 128 keys per tile: S = Q K^T  ->  P = exp2(S - m)  ->  O += P V
 //   attn_bwd_dkdv_ps_kernel   128 key rows: S^T = K Q^T, dP^T = V dO^T, dV += P^T dO, dK += dS^T Q
 //   attn_bwd_dq_ps_kernel     128 query rows: S = Q K^T, dP = dO V^T, dQ += dS K
+//   attn_fwd_tm_kernel, attn_fwd_split_kernel   forward of short rows of head size 128, two maxima per row (see kSplitRows)
 // Head size 128 also has earlier kernels with one CTA per work item, and with 64-wide tiles and P / dS in shared memory; they
 // run when MSAMP_ATTN_{FWD,BWD}_PERSIST=0 or MSAMP_ATTN_{FWD,BWD}_SMEM=1 and serve as a cross-check.
 //
@@ -16,9 +17,9 @@
 // The backward pass is deterministic (no atomics).  Every mbarrier wait is bounded; when one gives
 // up, bit 2 (value 4) of the device status word is set and the CTA frees its TMEM and returns.
 //
-// Head size 64 took the mma.sync kernels of attention.cu before: 8 x 1024 x 12 heads, causal, 78 + 274 us forward + backward,
-// now 42 + 109 us; 64 x 197 x 12 heads, 72 + 256 us, now 43 + 120 us.  Those kernels remain for views that a tensor map
-// cannot describe and as a cross-check (MSAMP_ATTN_IMPL=mma); from 33 keys on they are nowhere faster by more than 5 us.
+// Head size 64 took the mma.sync kernels of attention.cu before: 8 x 1024 x 12 heads, causal, 71 + 253 us forward + backward on
+// the device, now 44 + 107 us; 64 x 197 x 12 heads, 61 + 218 us, now 45 + 119 us.  Those kernels remain for views that a tensor map
+// cannot describe and as a cross-check (MSAMP_ATTN_IMPL=mma).
 #include <cstdlib>
 #include <mutex>
 #include <unordered_map>
@@ -592,7 +593,8 @@ attn_fwd_tm_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll
         for (int i = 0; i < 64; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(r[i >> 5][i & 31]));
       }
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sl;    // sl > 0
+      const float raw = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      const float mx = raw == -INFINITY ? -INFINITY : raw * sl;    // no visible key: whatever the sign of the scale
       const bool grow_m = mx > m + kRescaleStep || (m == -INFINITY && mx > -INFINITY);
       if (__any_sync(0xffffffffu, grow_m)) {
         const float m_new = grow_m ? mx : m;
@@ -680,6 +682,344 @@ attn_fwd_tm_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   if (warp == 1) tc5::tmem_dealloc(tmem_base, TM_COLS);
 }
 
+// ============================================== forward, head size 128, many short rows: attn_fwd_tm_kernel over a list of items
+namespace fwd2s {
+using namespace fwd2;    // same tiles, rings and tensor-memory layout
+constexpr uint32_t OFF_X3 = OFF_V + NV * TILE_V;          // two merge buffers of 2 KB (alternating work items)
+constexpr uint32_t OFF_BAR3 = OFF_X3 + 4096;
+enum { B3_QE = NBAR, B3_OE = NBAR + 1, B3_X = NBAR + 2, NBAR3 = NBAR + 3 };
+constexpr int SMEM3 = OFF_BAR3 + NBAR3 * 8 + 16 + 1024;
+}    // namespace fwd2s
+
+// Work item -> (level, batch * head) for the persistent attention kernels: groups of G heads, inside a group by rising
+// level (level 0 is the longest row), so that consecutive waves work on the same heads (their K / V or Q / dO stay in
+// L2) and a walk that alternates direction per wave gives every CTA the same amount of work per group.
+struct ItemOrder {
+  int n_lv, bh_total, G;
+  __device__ __forceinline__ void decode(int item, int& level, int& bh) const {
+    const int g = item / (G * n_lv);
+    const int hg = min(G, bh_total - g * G);
+    const int j = item - g * G * n_lv;
+    level = j / hg;
+    bh = g * G + j % hg;
+  }
+};
+
+// The schedule of attn_fwd_tm_kernel with one CTA per SM that walks the (query tile, batch * head) items.  Every ring (K, V, score
+// slots) and every barrier keeps running across items, so the TMA warp loads Q, K and V of the next item while the softmax warps
+// are still in the epilogue of the current one, and the MMA warp has the first two score tiles of the next item ready when they
+// return.  B3_QE: all score MMAs of an item are complete, the Q tile may be overwritten; B3_OE: the softmax warps have read both
+// accumulators, the first P V of the next item may overwrite them; B3_X: the eight softmax warps meet before the two groups'
+// partial results are merged.  Bound by the exponentials and the groups' waits for each other (attn_fwd_ps_kernel has neither
+// group wait, but one maximum per row instead of two: see the rule in msamp_attention_tc_fwd).
+__global__ void __launch_bounds__(kTcThreads, 1)
+attn_fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                   const __grid_constant__ CUtensorMap map_v, const TcParams p, int n_qt, int n_items) {
+  using namespace fwd2s;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_addr = tc5::smem_u32(smem_raw);
+  const uint32_t base = (raw_addr + 1023u) & ~1023u;
+  uint8_t* smem = smem_raw + (base - raw_addr);
+  const uint32_t bars = base + OFF_BAR3;
+  auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(smem + OFF_BAR3 + NBAR3 * 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
+  auto wait_warp = [&](uint32_t br, uint32_t ph) {
+    return __all_sync(0xffffffffu, tc5::mbar_wait(br, ph, abort_flag, p.status, kStatusBit)) != 0;
+  };
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int n_all = (p.seqlen + 63) / 64;
+  const ItemOrder order{n_qt, p.batch * p.heads, p.group};
+  const int n_waves = (n_items + (int)gridDim.x - 1) / (int)gridDim.x;
+  auto item_at = [&](int w) {
+    const int c = (w & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
+    return w * (int)gridDim.x + c;
+  };
+  auto item_tiles = [&](int qt) {
+    const int n_kv = p.causal ? min(2 * qt + 2, n_all) : n_all;
+    return (n_kv + 1) >> 1;
+  };
+
+  if (threadIdx.x == 0) {
+    tc5::mbar_init(bar(B_Q), 1);
+    for (int s = 0; s < NK; ++s) {
+      tc5::mbar_init(bar(B_KF + s), 1);
+      tc5::mbar_init(bar(B_KE + s), 1);
+    }
+    for (int s = 0; s < NV; ++s) {
+      tc5::mbar_init(bar(B_VF + s), 1);
+      tc5::mbar_init(bar(B_VE + s), 1);
+    }
+    tc5::mbar_init(bar(B_SF + 0), 1);
+    tc5::mbar_init(bar(B_SF + 1), 1);
+    for (int s = 0; s < 4; ++s) tc5::mbar_init(bar(B_PF + s), 4);
+    tc5::mbar_init(bar(B_OF + 0), 1);
+    tc5::mbar_init(bar(B_OF + 1), 1);
+    tc5::mbar_init(bar(B_ACC), 1);
+    tc5::mbar_init(bar(B3_QE), 1);
+    tc5::mbar_init(bar(B3_OE), 8);
+    tc5::mbar_init(bar(B3_X), 8);
+    *abort_flag = 0;
+    tc5::mbar_fence_init();
+    tc5::tma_prefetch_desc(&map_q);
+    tc5::tma_prefetch_desc(&map_k);
+    tc5::tma_prefetch_desc(&map_v);
+  }
+  if (warp == 1) {
+    tc5::tmem_alloc(tc5::smem_u32(tmem_holder), TM_COLS);
+    tc5::tmem_relinquish();
+  }
+  tc5::fence_before_sync();
+  __syncthreads();
+  tc5::fence_after_sync();
+  const uint32_t tmem_base = *tmem_holder;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      int gt = 0;    // 128-key tiles loaded so far (all items)
+      bool ok = true;
+      int it = 0;
+      for (int w = 0; w < n_waves && ok; ++w) {
+        const int item = item_at(w);
+        if (item >= n_items) continue;
+        int level, bh;
+        order.decode(item, level, bh);
+        const int qt = n_qt - 1 - level;
+        const int b = bh / p.heads, h = bh - b * p.heads;
+        const int n_t = item_tiles(qt);
+        if (it > 0 && !tc5::mbar_wait(bar(B3_QE), (uint32_t)(it - 1) & 1u, abort_flag, p.status, kStatusBit)) break;
+        tc5::mbar_arrive_expect_tx(bar(B_Q), TILE_Q);
+        tc5::tma_load_4d(base + OFF_Q, &map_q, 0, h, qt * 128, b, bar(B_Q));
+        tc5::tma_load_4d(base + OFF_Q + PANEL_Q, &map_q, 64, h, qt * 128, b, bar(B_Q));
+        for (int t = 0; t < n_t && ok; ++t, ++gt) {
+          const int ks = gt % NK;
+          if (!tc5::mbar_wait(bar(B_KE + ks), ((uint32_t)(gt / NK) & 1u) ^ 1u, abort_flag, p.status, kStatusBit)) { ok = false; break; }
+          tc5::mbar_arrive_expect_tx(bar(B_KF + ks), TILE_K);
+          tc5::tma_load_4d(base + OFF_K + ks * TILE_K, &map_k, 0, h, t * 128, b, bar(B_KF + ks));
+          tc5::tma_load_4d(base + OFF_K + ks * TILE_K + PANEL_K, &map_k, 64, h, t * 128, b, bar(B_KF + ks));
+          for (int g = 0; g < 2; ++g) {
+            const int gj = 2 * gt + g;    // 64-key sub-tiles loaded so far
+            const int vs = gj % NV;
+            if (!tc5::mbar_wait(bar(B_VE + vs), ((uint32_t)(gj / NV) & 1u) ^ 1u, abort_flag, p.status, kStatusBit)) { ok = false; break; }
+            tc5::mbar_arrive_expect_tx(bar(B_VF + vs), TILE_V);
+            tc5::tma_load_4d(base + OFF_V + vs * TILE_V, &map_v, 0, h, (2 * t + g) * 64, b, bar(B_VF + vs));
+            tc5::tma_load_4d(base + OFF_V + vs * TILE_V + PANEL_V, &map_v, 64, h, (2 * t + g) * 64, b, bar(B_VF + vs));
+          }
+        }
+        ++it;
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      const uint32_t idesc_s = tc5::idesc_bf16(128, 128, 0, 0);
+      const uint32_t idesc_o = tc5::idesc_bf16(128, 128, 0, 1);
+      auto issue_s = [&](int gs) -> bool {    // S[gs & 1] = Q K^T for the gs-th tile of this CTA
+        const int ks = gs % NK;
+        if (!tc5::mbar_wait(bar(B_KF + ks), (uint32_t)(gs / NK) & 1u, abort_flag, p.status, kStatusBit)) return false;
+        tc5::fence_after_sync();
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) {
+          const uint32_t off = (uint32_t)(kk >> 2) * PANEL_Q + (uint32_t)(kk & 3) * 32u;
+          tc5::mma_f16(tmem_base + TM_S + (uint32_t)(gs & 1) * 128u, tc5::smem_desc_k_sw128(base + OFF_Q + off),
+                       tc5::smem_desc_k_sw128(base + OFF_K + ks * TILE_K + off), idesc_s, kk ? 1u : 0u);
+        }
+        tc5::mma_commit(bar(B_KE + ks));
+        tc5::mma_commit(bar(B_SF + (gs & 1)));
+        return true;
+      };
+      int g0 = 0;    // tiles of earlier items
+      bool ok = true;
+      int it = 0;
+      for (int w = 0; w < n_waves && ok; ++w) {
+        const int item = item_at(w);
+        if (item >= n_items) continue;
+        int level, bh;
+        order.decode(item, level, bh);
+        const int n_t = item_tiles(n_qt - 1 - level);
+        if (!tc5::mbar_wait(bar(B_Q), (uint32_t)it & 1u, abort_flag, p.status, kStatusBit)) { ok = false; break; }
+        for (int t = 0; t < 2 && t < n_t; ++t)
+          if (!issue_s(g0 + t)) { ok = false; break; }
+        if (!ok) break;
+        if (n_t <= 2) tc5::mma_commit(bar(B3_QE));    // every score product of this item has been issued
+        // the softmax warps must have read the previous item's accumulators before they are overwritten
+        if (it > 0 && !tc5::mbar_wait(bar(B3_OE), (uint32_t)(it - 1) & 1u, abort_flag, p.status, kStatusBit)) { ok = false; break; }
+        for (int t = 0; t < n_t && ok; ++t) {
+          const int gs = g0 + t;
+          for (int g = 0; g < 2; ++g) {
+            const int gj = 2 * gs + g;
+            const int vs = gj % NV;
+            // the data barrier first: a wait costs 100+ cycles even when its phase completed long ago, and this one
+            // then passes while the softmax warps are still at work on P
+            if (!tc5::mbar_wait(bar(B_VF + vs), (uint32_t)(gj / NV) & 1u, abort_flag, p.status, kStatusBit)) { ok = false; break; }
+            if (!tc5::mbar_wait(bar(B_PF + (gs & 1) * 2 + g), (uint32_t)(gs >> 1) & 1u, abort_flag, p.status, kStatusBit)) { ok = false; break; }
+            tc5::fence_after_sync();
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+              tc5::mma_f16_ta(tmem_base + TM_O + (uint32_t)g * 128u,
+                              tmem_base + TM_S + (uint32_t)(gs & 1) * 128u + (uint32_t)g * 64u + (uint32_t)kk * 8u,
+                              tc5::smem_desc_mn_sw128(base + OFF_V + vs * TILE_V + (uint32_t)kk * 2048u, PANEL_V), idesc_o,
+                              (t > 0 || kk) ? 1u : 0u);
+            }
+            tc5::mma_commit(bar(B_VE + vs));
+            tc5::mma_commit(bar(B_OF + g));
+          }
+          if (ok && t + 2 < n_t) {
+            if (!issue_s(gs + 2)) { ok = false; break; }
+            if (t + 3 == n_t) tc5::mma_commit(bar(B3_QE));
+          }
+        }
+        if (ok) tc5::mma_commit(bar(B_ACC));
+        g0 += n_t;
+        ++it;
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ softmax: one thread per query row and group
+    const int qd = warp & 3;           // TMEM lane quarter this warp may access
+    const int wg = (warp - 2) >> 2;    // group g: second index of the 64-key halves it owns
+    const int row = qd * 32 + lane;
+    const uint32_t tlane = tmem_base + ((uint32_t)(qd * 32) << 16);
+    const uint32_t to = tlane + TM_O + (uint32_t)wg * 128u;
+    const float sl = p.scale * kLog2e;
+    int g0 = 0;
+    bool ok = true;
+    int it = 0;
+    for (int w = 0; w < n_waves; ++w) {
+      const int item = item_at(w);
+      if (item >= n_items) continue;
+      int level, bh;
+      order.decode(item, level, bh);
+      const int qt = n_qt - 1 - level;
+      const int b = bh / p.heads, h = bh - b * p.heads;
+      const int n_t = item_tiles(qt);
+      const int q0 = qt * 128;
+      const int grow = q0 + row;
+      const int lim = p.causal ? min(grow, p.seqlen - 1) : p.seqlen - 1;    // last visible column
+      float m = -INFINITY, l = 0.0f;    // reference maximum (log2 units) and row sum of this group
+      for (int t = 0; t < n_t; ++t) {
+        const int gs = g0 + t;
+        const uint32_t ts = tlane + TM_S + (uint32_t)(gs & 1) * 128u + (uint32_t)wg * 64u;
+        if (!wait_warp(bar(B_SF + (gs & 1)), (uint32_t)(gs >> 1) & 1u)) { ok = false; break; }
+        tc5::fence_after_sync();
+        uint32_t r[2][32];
+        tc5::tmem_ld32(ts, r[0]);
+        tc5::tmem_ld32(ts + 32u, r[1]);
+        tc5::tmem_ld_wait();
+        const int col0 = (2 * t + wg) * 64;
+        const bool need_mask = (p.causal && col0 + 63 > q0) || (col0 + 64 > p.seqlen);
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        if (need_mask) {
+#pragma unroll
+          for (int i = 0; i < 64; ++i)
+            if (col0 + i <= lim) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(r[i >> 5][i & 31]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(r[i >> 5][i & 31]));
+        }
+        const float raw = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+        const float mx = raw == -INFINITY ? -INFINITY : raw * sl;
+        const bool grow_m = mx > m + kRescaleStep || (m == -INFINITY && mx > -INFINITY);
+        if (__any_sync(0xffffffffu, grow_m)) {
+          const float m_new = grow_m ? mx : m;
+          const float corr = (m == -INFINITY) ? 0.0f : ex2(m - m_new);
+          if (t > 0) {
+            // every earlier product of this group and item must have landed in O before it is rescaled
+            if (!wait_warp(bar(B_OF + wg), (uint32_t)(gs - 1) & 1u)) { ok = false; break; }
+            tc5::fence_after_sync();
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+              uint32_t x[32];
+              tc5::tmem_ld32(to + (uint32_t)c * 32u, x);
+              tc5::tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) x[i] = __float_as_uint(__uint_as_float(x[i]) * corr);
+              tc5::tmem_st32(to + (uint32_t)c * 32u, x);
+            }
+          }
+          l *= corr;
+          m = m_new;
+        }
+        const float m_use = (m == -INFINITY) ? 0.0f : m;
+        float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        uint32_t pk[32];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {    // columns 8g .. 8g+7 -> packed columns 4g .. 4g+3
+          float e[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            e[i] = ex2(fmaf(__uint_as_float(r[g >> 2][(g & 3) * 8 + i]), sl, -m_use));
+            if (need_mask && col0 + g * 8 + i > lim) e[i] = 0.0f;
+            sum4[i & 3] += e[i];
+          }
+          pk[4 * g] = pack_bf16(e[0], e[1]);
+          pk[4 * g + 1] = pack_bf16(e[2], e[3]);
+          pk[4 * g + 2] = pack_bf16(e[4], e[5]);
+          pk[4 * g + 3] = pack_bf16(e[6], e[7]);
+        }
+        l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+        tc5::tmem_st32(ts, pk);
+        tc5::tmem_st_wait();    // also covers the rescaled accumulator
+        tc5::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc5::mbar_arrive(bar(B_PF + (gs & 1) * 2 + wg));
+      }
+      ok = ok && wait_warp(bar(B_ACC), (uint32_t)it & 1u);
+      tc5::fence_after_sync();
+      // merge the two groups through shared memory (two buffers, alternating items: a warp that is already in the next
+      // item's merge cannot overwrite values another warp still reads)
+      float* xm = reinterpret_cast<float*>(smem + OFF_X3 + (uint32_t)(it & 1) * 2048u);    // [2][128] maxima, then [2][128] sums
+      float* xl = xm + 256;
+      if (!ok) break;
+      xm[wg * 128 + row] = m;
+      xl[wg * 128 + row] = l;
+      // the eight warps meet on an mbarrier (bounded wait) rather than on a named barrier: a warp that gave up on an
+      // earlier wait leaves without arriving, and the others then give up here instead of waiting for it for ever
+      __syncwarp();
+      if (lane == 0) tc5::mbar_arrive(bar(B3_X));
+      if (!wait_warp(bar(B3_X), (uint32_t)it & 1u)) { ok = false; break; }
+      const float m0 = xm[row], m1 = xm[128 + row], l0 = xl[row], l1 = xl[128 + row];
+      const float mm = fmaxf(m0, m1);
+      const float f0 = (m0 == -INFINITY) ? 0.0f : ex2(m0 - mm);
+      const float f1 = (m1 == -INFINITY) ? 0.0f : ex2(m1 - mm);
+      const float lt = l0 * f0 + l1 * f1;
+      const float inv = lt > 0.0f ? 1.0f / lt : 0.0f;
+      const float gg0 = f0 * inv, gg1 = f1 * inv;
+      uint32_t a0[2][32], a1[2][32];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        tc5::tmem_ld32(tlane + TM_O + (uint32_t)wg * 64u + (uint32_t)c * 32u, a0[c]);
+        tc5::tmem_ld32(tlane + TM_O + 128u + (uint32_t)wg * 64u + (uint32_t)c * 32u, a1[c]);
+      }
+      tc5::tmem_ld_wait();
+      tc5::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc5::mbar_arrive(bar(B3_OE));    // the accumulators may take the next item
+      __nv_bfloat16* dst = p.o + (int64_t)b * p.o_sb + (int64_t)grow * p.o_ss + (int64_t)h * p.o_sh + wg * 64;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        float v[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = fmaf(__uint_as_float(a1[c][i]), gg1, __uint_as_float(a0[c][i]) * gg0);
+        if (grow < p.seqlen) st_row32(dst + c * 32, v);
+      }
+      if (wg == 0 && grow < p.seqlen) p.lse[(int64_t)bh * p.seqlen + grow] = lt > 0.0f ? mm * kLn2 + logf(lt) : -INFINITY;
+      g0 += n_t;
+      ++it;
+    }
+  }
+
+  // ---------------------------------------------------------------------- tear-down
+  __syncwarp();
+  if (*abort_flag) __nanosleep(200000);    // let copies / MMAs in flight finish before smem and TMEM go away
+  tc5::fence_before_sync();
+  __syncthreads();
+  tc5::fence_after_sync();
+  if (warp == 1) tc5::tmem_dealloc(tmem_base, TM_COLS);
+}
+
 // ================================================================= forward, persistent CTAs over (query tile, batch, head)
 // Thread layout of the persistent kernels: one warpgroup of which warp 0 issues TMA and warp 1 the MMAs, and two warpgroups
 // of softmax threads.  The register file is split by setmaxnreg: AUX for the first, (384 * 168 - 128 * AUX) / 256 for the
@@ -709,6 +1049,7 @@ constexpr uint32_t PANEL = 128 * 128;    // [128 rows][64 bf16]: one 64-wide sli
 template <int D>
 struct Cfg {
   static constexpr int HP = D / 64;
+  static constexpr int NA = D == 128 ? 1 : 2;    // running maxima, row sums and accumulators of a row, one per 128 / NA columns of a tile
   static constexpr int NK = D == 128 ? 3 : 4, NV = D == 128 ? 2 : 4;    // ring depths of the K and V tiles (128 keys each)
   static constexpr uint32_t TILE = HP * PANEL;
   static constexpr uint32_t OFF_K = 2 * TILE, OFF_V = OFF_K + NK * TILE, OFF_BAR = OFF_V + NV * TILE;    // two Q tiles first
@@ -717,10 +1058,11 @@ struct Cfg {
   static constexpr int SMEM = OFF_BAR + NBAR * 8 + 16 + 1024;
   static_assert(SMEM <= 227 * 1024, "persistent forward kernel: shared memory");
 };
-// scores (128 columns), P of each group (64), output of each group (D)
+// scores (128 columns), P of each group (64), accumulators of each group (NA * D = 128)
 constexpr int kFwdAux = 72;    // registers of the TMA and MMA threads
 constexpr uint32_t TM_S = 0, TM_P = 128, TM_O = 256, TM_COLS = 512;
-constexpr float kRescaleStep = 8.0f;    // the reference maximum may lag the true one by 2^8
+constexpr int kExactTiles = 4;          // head size 128: the maximum is exact for the first tiles of a row, then it may
+constexpr float kRescaleStep = 4.0f;    // lag the true one by 2^4
 }    // namespace fwd3
 
 // Work item (query tile, batch * head) lists of the forward kernel.  Stream g of CTA c is worker g * CTAs + c and takes one
@@ -808,6 +1150,13 @@ struct FwdSeq {
 // What bounds it, per tile of 128 x 128: 1024 cycles of MUFU (16384 exponentials at 16 a clock), 12 to 16 MMAs of about 70
 // cycles (a 128 x N x 16 bf16 MMA costs that for N = 64 and for N = 128: the 4 KB A operand is fed at 64 B/clk), and some
 // 1200 cycles of maxima, sums, packing and TMEM traffic of one group, which only the other group's exponentials hide.
+//  * P is relative to the row's running maximum, so that the largest probability is exactly 1 and rounds to bf16 without error: with a
+//    reference that lagged by up to 2^8 the output of peaked rows was up to 20 % further from 64 bits (scores of standard deviation
+//    2, 2048 keys of 64).  Head size 64 has tensor memory for two accumulators per row and takes a maximum per 64 keys, as a 64-key
+//    tile would: never further off than the mma.sync kernels (64 x 197 rows: 0.00212 against 0.00215).  Head size 128 has one, exact
+//    over the first kExactTiles tiles of a row; later the weights are spread, and a lag of 2^4 saves most rescales (2 % of the time
+//    at 2048 and 4096 rows).  The exact maximum costs 7 % of the time at 64 (8 x 1024 x 12 heads, causal: 41 -> 43.5 us) and 3 % at
+//    128; a rescale moves all columns through registers at once.
 //  * A group reads its 128 scores into registers and releases the one score slot at once, so that the scores of the next
 //    tile (the other group's) are there before they are needed; P goes to a place of its own, from where O_g += P V reads
 //    it as a TMEM operand.  When P was written over the scores, a group waited 1500 of 3950 cycles per tile for its next
@@ -817,8 +1166,8 @@ struct FwdSeq {
 //  * The tensor pipe buffers next to nothing and a wait or a commit costs the issuing thread 50 to 250 cycles, so one thread
 //    that issued both products kept the pipe idle for half of the tile.  Two threads of two warps issue them; nothing
 //    depends on the order between the two, every reuse below is a barrier.  Both probe their next tile while MMAs run.
-// Measured, forward only: 4 x 2048 x 32 heads of 128, causal, 211 -> 191 us; 2 x 4096 x 16 heads of 128, causal, 232 -> 177 us;
-// 8 x 1024 x 12 heads of 64, causal, 78 us (mma.sync) -> 42 us; 64 x 197 x 12 heads of 64, 72 us (mma.sync) -> 43 us.
+// Measured, forward only, against one stream of tiles that both groups split: 4 x 2048 x 32 heads of 128, causal, 204 -> 190 to
+// 194 us; 2 x 4096 x 16 heads of 128, causal, 242 -> 208 us; 1 x 8192 x 16, 433 -> 328 us.
 // Reuse: Q_g after the last score product of its item (B_QE); the score slot after B_SE (tiles in sequence order); P_g and
 // the accumulator after P V of the group's previous tile (B_OF); the accumulator of a finished item is read before the group
 // hands over its next P (B_PF), so the next item's first product cannot overtake it.
@@ -828,7 +1177,7 @@ attn_fwd_ps_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                    const __grid_constant__ CUtensorMap map_v, const TcParams p, int n_qt, int n_items) {
   using namespace fwd3;
   using C = Cfg<D>;
-  constexpr int HP = C::HP, NK = C::NK, NV = C::NV;
+  constexpr int HP = C::HP, NK = C::NK, NV = C::NV, NA = C::NA;
   constexpr uint32_t TILE = C::TILE, OFF_Q = 0, OFF_K = C::OFF_K, OFF_V = C::OFF_V;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = tc5::smem_u32(smem_raw);
@@ -965,8 +1314,10 @@ attn_fwd_ps_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         tc5::fence_after_sync();
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
-          tc5::mma_f16_ta(tmem_base + TM_O + (uint32_t)(g * D), tmem_base + TM_P + (uint32_t)g * 64u + (uint32_t)kk * 8u,
-                          tc5::smem_desc_mn_sw128(base + OFF_V + vr.slot * TILE + (uint32_t)kk * 2048u, PANEL), idesc, (!first || kk) ? 1u : 0u);
+          const int a = kk / (8 / NA);    // accumulator of these 16 keys
+          tc5::mma_f16_ta(tmem_base + TM_O + (uint32_t)(g * 128 + a * D), tmem_base + TM_P + (uint32_t)g * 64u + (uint32_t)kk * 8u,
+                          tc5::smem_desc_mn_sw128(base + OFF_V + vr.slot * TILE + (uint32_t)kk * 2048u, PANEL), idesc,
+                          (!first || kk % (8 / NA)) ? 1u : 0u);
         }
         tc5::mma_commit(bar(C::B_OF + g));
         tc5::mma_commit(bar(C::B_VE + vr.slot));
@@ -981,7 +1332,7 @@ attn_fwd_ps_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     const int wg = (warp - 4) >> 2;    // stream
     const int row = qd * 32 + lane;
     const uint32_t tlane = tmem_base + ((uint32_t)(qd * 32) << 16);
-    const uint32_t ts = tlane + TM_S, tp = tlane + TM_P + (uint32_t)wg * 64u, to = tlane + TM_O + (uint32_t)(wg * D);
+    const uint32_t ts = tlane + TM_S, tp = tlane + TM_P + (uint32_t)wg * 64u, to = tlane + TM_O + (uint32_t)wg * 128u;
     const float sl = p.scale * kLog2e;
     const uint64_t sl2 = f2_pack(sl, sl);
     uint32_t n = 0;    // tiles of this stream so far
@@ -995,7 +1346,12 @@ attn_fwd_ps_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       const int grow = q0 + row;
       const int lim = p.causal ? min(grow, p.seqlen - 1) : p.seqlen - 1;    // last visible column
       const int wlim = p.causal ? min(q0 + qd * 32 + 31, p.seqlen - 1) : p.seqlen - 1;    // the same for the warp's last row
-      float m = -INFINITY, l = 0.0f;    // reference maximum (log2 units) and row sum
+      float m[NA], l[NA];    // running maximum (log2 units) and row sum
+#pragma unroll
+      for (int a = 0; a < NA; ++a) {
+        m[a] = -INFINITY;
+        l[a] = 0.0f;
+      }
       for (int t = item.first; t < n_t; t += item.step, ++n) {
         if (!wait_warp(bar(C::B_SF + wg), n & 1u)) { ok = false; break; }
         tc5::fence_after_sync();
@@ -1011,42 +1367,53 @@ attn_fwd_ps_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // 32-column chunks in which any row of this warp sees a key
         const int nch = need_mask ? min(4, (wlim - col0) / 32 + 1) : 4;
         const int rel = lim - col0;    // last visible column of this row
-        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};    // 4 / NA partial maxima for each accumulator
         if (need_mask) {
 #pragma unroll
           for (int c = 0; c < 4; ++c)
             if (c < nch) {
 #pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (c * 32 + i <= rel) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(r[c][i]));
+              for (int i = 0; i < 32; ++i) {
+                float& x = mx4[NA == 1 ? i & 3 : (c >> 1) * 2 + (i & 1)];
+                if (c * 32 + i <= rel) x = fmaxf(x, __uint_as_float(r[c][i]));
+              }
             }
         } else {
 #pragma unroll
           for (int c = 0; c < 4; ++c)
 #pragma unroll
-            for (int i = 0; i < 32; i += 2)
-              mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], __uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1]));
+            for (int i = 0; i < 32; i += 2) {
+              float& x = mx4[NA == 1 ? (i >> 1) & 3 : (c >> 1) * 2 + ((i >> 1) & 1)];
+              x = max3(x, __uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1]));
+            }
         }
-        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sl;    // sl > 0
-        const bool grow_m = mx > m + kRescaleStep || (m == -INFINITY && mx > -INFINITY);
-        float corr = 1.0f;
-        const bool rescale = __any_sync(0xffffffffu, grow_m);
-        if (rescale) {
-          const float m_new = grow_m ? mx : m;
-          corr = (m == -INFINITY) ? 0.0f : ex2(m - m_new);
-          l *= corr;
-          m = m_new;
+        const float lag = NA == 1 && t >= item.first + kExactTiles * item.step ? kRescaleStep : 0.0f;
+        float corr[NA];
+        bool rescale[NA];
+        uint64_t nm2[NA];
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+          const float raw = NA == 1 ? fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) : fmaxf(mx4[2 * a], mx4[2 * a + 1]);
+          const float mx = raw == -INFINITY ? -INFINITY : raw * sl;    // no visible key: whatever the sign of the scale
+          const bool grow_m = mx > m[a] + lag || (m[a] == -INFINITY && mx > -INFINITY);
+          corr[a] = 1.0f;
+          rescale[a] = __any_sync(0xffffffffu, grow_m);
+          if (grow_m) {
+            corr[a] = (m[a] == -INFINITY) ? 0.0f : ex2(m[a] - mx);
+            l[a] *= corr[a];
+            m[a] = mx;
+          }
+          const float m_use = (m[a] == -INFINITY) ? 0.0f : m[a];
+          nm2[a] = f2_pack(-m_use, -m_use);
         }
-        const float m_use = (m == -INFINITY) ? 0.0f : m;
         // p = exp2(s * sl - m), two columns per multiply-add and per sum; masked columns are cleared afterwards
-        const uint64_t nm2 = f2_pack(-m_use, -m_use);
         uint64_t sum2[2] = {f2_pack(0.0f, 0.0f), f2_pack(0.0f, 0.0f)};
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           if (c < nch) {
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
-              const float2 x = f2_unpack(f2_fma(f2_pack(__uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1])), sl2, nm2));
+              const float2 x = f2_unpack(f2_fma(f2_pack(__uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1])), sl2, nm2[c * NA / 4]));
               r[c][i] = __float_as_uint(ex2(x.x));
               r[c][i + 1] = __float_as_uint(ex2(x.y));
             }
@@ -1063,26 +1430,43 @@ attn_fwd_ps_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
             const float e0 = __uint_as_float(r[c][i]), e1 = __uint_as_float(r[c][i + 1]);
-            sum2[(i >> 1) & 1] = f2_add(sum2[(i >> 1) & 1], f2_pack(e0, e1));
+            uint64_t& x = sum2[NA == 1 ? (i >> 1) & 1 : c >> 1];
+            x = f2_add(x, f2_pack(e0, e1));
             r[c >> 1][(c & 1) * 16 + (i >> 1)] = pack_bf16(e0, e1);
           }
         }
         const float2 sa = f2_unpack(sum2[0]), sb = f2_unpack(sum2[1]);
-        l += (sa.x + sa.y) + (sb.x + sb.y);
+        if (NA == 1) {
+          l[0] += (sa.x + sa.y) + (sb.x + sb.y);
+        } else {
+          l[0] += sa.x + sa.y;
+          l[NA - 1] += sb.x + sb.y;
+        }
         // P V of this group's previous tile is complete: P may be overwritten, O may be rescaled
         if (n > 0 && !wait_warp(bar(C::B_OF + wg), (n - 1) & 1u)) { ok = false; break; }
         tc5::fence_after_sync();
         tc5::tmem_st32(tp, r[0]);
         tc5::tmem_st32(tp + 32u, r[1]);
-        if (rescale && t > item.first) {
-#pragma unroll 1
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t x[32];
-            tc5::tmem_ld32(to + (uint32_t)c * 32u, x);
-            tc5::tmem_ld_wait();
+        if (t > item.first) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) x[i] = __float_as_uint(__uint_as_float(x[i]) * corr);
-            tc5::tmem_st32(to + (uint32_t)c * 32u, x);
+          for (int a = 0; a < NA; ++a) {
+            if (rescale[a]) {
+              const uint64_t c2 = f2_pack(corr[a], corr[a]);
+              uint32_t x[D / 32][32];    // all columns at once: one round trip to tensor memory
+#pragma unroll
+              for (int c = 0; c < D / 32; ++c) tc5::tmem_ld32(to + (uint32_t)(a * D + c * 32), x[c]);
+              tc5::tmem_ld_wait();
+#pragma unroll
+              for (int c = 0; c < D / 32; ++c) {
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) {
+                  const float2 v = f2_unpack(f2_mul(f2_pack(__uint_as_float(x[c][i]), __uint_as_float(x[c][i + 1])), c2));
+                  x[c][i] = __float_as_uint(v.x);
+                  x[c][i + 1] = __float_as_uint(v.y);
+                }
+                tc5::tmem_st32(to + (uint32_t)(a * D + c * 32), x[c]);
+              }
+            }
           }
         }
         tc5::tmem_st_wait();
@@ -1095,24 +1479,37 @@ attn_fwd_ps_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       const int64_t lse_row = (int64_t)bh * p.seqlen + grow;
       __nv_bfloat16* dst = p.o + (int64_t)b * p.o_sb + (int64_t)(q0 + qd * 32) * p.o_ss + (int64_t)h * p.o_sh;    // the warp's first row
       const int rows = p.seqlen - q0 - qd * 32;    // of which exist
+      // the row's maximum and sum over its accumulators, and the factor of each
+      float mr = m[0], lr = l[0], f[NA];
+      f[0] = 1.0f;
+      if (NA == 2) {
+        mr = fmaxf(m[0], m[NA - 1]);
+        f[0] = (m[0] == -INFINITY) ? 0.0f : ex2(m[0] - mr);
+        f[NA - 1] = (m[NA - 1] == -INFINITY) ? 0.0f : ex2(m[NA - 1] - mr);
+        lr = l[0] * f[0] + l[NA - 1] * f[NA - 1];
+      }
       if (!item.shared) {
-        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+        const float inv = lr > 0.0f ? 1.0f / lr : 0.0f;
 #pragma unroll
         for (int c = 0; c < D; c += 64) {
-          uint32_t a[2][32];
-          tc5::tmem_ld32(to + (uint32_t)c, a[0]);
-          tc5::tmem_ld32(to + (uint32_t)c + 32u, a[1]);
-          tc5::tmem_ld_wait();
           float v[64];
 #pragma unroll
-          for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(a[i >> 5][i & 31]) * inv;
+          for (int a = 0; a < NA; ++a) {
+            uint32_t x[2][32];
+            tc5::tmem_ld32(to + (uint32_t)(a * D + c), x[0]);
+            tc5::tmem_ld32(to + (uint32_t)(a * D + c) + 32u, x[1]);
+            tc5::tmem_ld_wait();
+            const float fa = f[a] * inv;
+#pragma unroll
+            for (int i = 0; i < 64; ++i) v[i] = a ? fmaf(__uint_as_float(x[i >> 5][i & 31]), fa, v[i]) : __uint_as_float(x[i >> 5][i & 31]) * fa;
+          }
           st_rows64(dst + c, p.o_ss, rows, v);
         }
         tc5::fence_before_sync();    // the next item's first P is handed over after these reads
-        if (grow < p.seqlen) p.lse[lse_row] = l > 0.0f ? m * kLn2 + logf(l) : -INFINITY;
+        if (grow < p.seqlen) p.lse[lse_row] = lr > 0.0f ? mr * kLn2 + logf(lr) : -INFINITY;
       } else {
-        // the last item of the CTA: maxima and sums change hands through the P columns, which nothing uses any more
-        uint32_t x[16] = {__float_as_uint(m), __float_as_uint(l)}, y[16];
+        // the last item of the CTA: maxima, sums and factors change hands through the P columns, which nothing uses any more
+        uint32_t x[16] = {__float_as_uint(mr), __float_as_uint(lr), __float_as_uint(f[0]), __float_as_uint(f[NA - 1])}, y[16];
         tc5::tmem_st16(tp, x);
         tc5::tmem_st_wait();
         tc5::fence_before_sync();
@@ -1123,24 +1520,31 @@ attn_fwd_ps_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         tc5::tmem_ld16(tlane + TM_P + (uint32_t)(wg ^ 1) * 64u, y);
         tc5::tmem_ld_wait();
         const float om = __uint_as_float(y[0]), ol = __uint_as_float(y[1]);
-        const float m0 = wg ? om : m, m1 = wg ? m : om, l0 = wg ? ol : l, l1 = wg ? l : ol;
+        const float m0 = wg ? om : mr, m1 = wg ? mr : om, l0 = wg ? ol : lr, l1 = wg ? lr : ol;
         const float mm = fmaxf(m0, m1);
         const float f0 = (m0 == -INFINITY) ? 0.0f : ex2(m0 - mm);
         const float f1 = (m1 == -INFINITY) ? 0.0f : ex2(m1 - mm);
         const float lt = l0 * f0 + l1 * f1;
         const float inv = lt > 0.0f ? 1.0f / lt : 0.0f;
-        const float gg0 = f0 * inv, gg1 = f1 * inv;
-        // each group stores every other 32 columns; an item of one tile has left the second accumulator unwritten
+        // each group stores every other 32 columns; an item of one tile has left the second stream's accumulators unwritten
 #pragma unroll
         for (int c = 0; c < D; c += 64) {
           const uint32_t col = (uint32_t)(c + wg * 32);
-          uint32_t a0[32], a1[32];
-          tc5::tmem_ld32(tlane + TM_O + col, a0);
-          tc5::tmem_ld32(tlane + TM_O + (uint32_t)D + col, a1);
-          tc5::tmem_ld_wait();
           float v[32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = fmaf(n_t > 1 ? __uint_as_float(a1[i]) : 0.0f, gg1, __uint_as_float(a0[i]) * gg0);
+          for (int a = 0; a < NA; ++a) {
+            const float own = f[a], others = __uint_as_float(y[a ? 3 : 2]);
+            const float g0 = f0 * inv * (wg ? others : own), g1 = f1 * inv * (wg ? own : others);
+            uint32_t a0[32], a1[32];
+            tc5::tmem_ld32(tlane + TM_O + (uint32_t)(a * D) + col, a0);
+            tc5::tmem_ld32(tlane + TM_O + 128u + (uint32_t)(a * D) + col, a1);
+            tc5::tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const float o0 = __uint_as_float(a0[i]) * g0;
+              v[i] = fmaf(n_t > 1 ? __uint_as_float(a1[i]) : 0.0f, g1, a ? v[i] + o0 : o0);
+            }
+          }
           if (row < p.seqlen - q0) st_row32(dst + (int64_t)lane * p.o_ss + col, v);
         }
         if (wg == 0 && grow < p.seqlen) p.lse[lse_row] = lt > 0.0f ? mm * kLn2 + logf(lt) : -INFINITY;
@@ -2219,20 +2623,6 @@ struct Cfg {
 };
 }    // namespace dqk3
 
-// Work item -> (level, batch * head) for the persistent attention kernels: groups of G heads, inside a group by rising
-// level (level 0 is the longest row), so that consecutive waves work on the same heads (their K / V or Q / dO stay in
-// L2) and a walk that alternates direction per wave gives every CTA the same amount of work per group.
-struct ItemOrder {
-  int n_lv, bh_total, G;
-  __device__ __forceinline__ void decode(int item, int& level, int& bh) const {
-    const int g = item / (G * n_lv);
-    const int hg = min(G, bh_total - g * G);
-    const int j = item - g * G * n_lv;
-    level = j / hg;
-    bh = g * G + j % hg;
-  }
-};
-
 // attn_bwd_dq_tm_kernel with one CTA per SM walking the (query tile, batch * head) items, the exponentials taken before dP is
 // waited for, the next K and V tile probed while MMAs run, and dQ stored in whole lines: 4 x 2048 x 32 heads of 128, causal,
 // 235 -> 206 us.  Rings, the score tile and
@@ -3050,6 +3440,15 @@ extern "C" int msamp_attention_fwd(const void*, const void*, const void*, void*,
 extern "C" int msamp_attention_bwd(const void*, const void*, const void*, const void*, const float*, const void*, void*, void*, void*, float*,
                                    const int64_t*, int, int, int, int, float, int, void*);
 
+// Head size 128, up to this many rows: the kernels that give each half of the 128 keys of a tile a maximum and an accumulator of its
+// own, attn_fwd_tm_kernel while the items fit the SMs once (its prologue is shorter: 12 heads of 200, 8.0 -> 7.2 us against
+// attn_fwd_split_kernel) and attn_fwd_split_kernel for longer lists.  attn_fwd_ps_kernel is up to 1.5 times as fast there (768 heads of
+// 128: 20 against 30 us), but has room for one accumulator only.  Its P is then relative to the maximum of all 128 keys, one
+// probability that is exactly 1 instead of two, and with few tiles the output is further from 64 bits: 0.00216 against 0.00210 at
+// 128 rows (relative 2-norm, of it 0.0017 from rounding the output), equal from 385 to 450 rows on, closer beyond (0.00220 against
+// 0.00227 at 384, not causal).  Up to 64 rows the two are the same.
+constexpr int kSplitRows = 448;
+
 // Same contract as msamp_attention_fwd (attention.cu), head_dim 64 or 128: strides are the (batch, seq, head)
 // element strides of q, k, v, o; every pointer 16-byte aligned, every stride a multiple of 8 elements.
 // All checks and tensor maps come before the first launch, so that a call that is refused has queued nothing.
@@ -3065,8 +3464,16 @@ MSAMP_API int msamp_attention_tc_fwd(const void* q, const void* k, const void* v
   // tiles, P in tensor memory), MSAMP_ATTN_FWD_PERSIST=0 one CTA per (query tile, batch, head) instead of persistent CTAs.
   static const bool smem_env = [] { const char* e = getenv("MSAMP_ATTN_FWD_SMEM"); return e && e[0] == '1'; }();
   static const bool persist_env = [] { const char* e = getenv("MSAMP_ATTN_FWD_PERSIST"); return !(e && e[0] == '0'); }();
-  const bool smem_operands = smem_env && head_dim == 128, persistent = persist_env || head_dim == 64;
-  const int k_rows = smem_operands ? 64 : 128, v_rows = !smem_operands && persistent ? 128 : 64;
+  const int n_qt = (seqlen + 127) / 128;
+  const int n_items = n_qt * batch * heads;
+  const int ctas = n_items < msamp_sm_count() ? n_items : msamp_sm_count();
+  enum { SMEM, TM, SPLIT, PS } kind = PS;
+  if (head_dim == 128) {
+    if (smem_env) kind = SMEM;
+    else if (!persist_env || (seqlen <= kSplitRows && n_items <= ctas)) kind = TM;
+    else if (seqlen > 64 && seqlen <= kSplitRows) kind = SPLIT;
+  }
+  const int k_rows = kind == SMEM ? 64 : 128, v_rows = kind == PS ? 128 : 64;
   CUtensorMap mq, mk, mv;
   int rc;
   if ((rc = make_map4(q, batch, heads, seqlen, head_dim, strides[0], strides[1], strides[2], 128, &mq))) return rc;
@@ -3079,20 +3486,22 @@ MSAMP_API int msamp_attention_tc_fwd(const void* q, const void* k, const void* v
   p.status = msamp_device_status_ptr();
   p.group = item_group(seqlen, head_dim);
   cudaStream_t stream = (cudaStream_t)stream_;
-  const int n_qt = (seqlen + 127) / 128;
   dim3 grid(n_qt, batch * heads);
-  if (smem_operands) {
+  if (kind == SMEM) {
     if ((rc = set_smem(attn_fwd_tc_kernel, fwd::SMEM))) return rc;
     attn_fwd_tc_kernel<<<grid, kTcThreads, fwd::SMEM, stream>>>(mq, mk, mv, p);
     return msamp_check_launch("attn_fwd_tc_kernel");
   }
-  if (!persistent) {
+  if (kind == TM) {
     if ((rc = set_smem(attn_fwd_tm_kernel, fwd2::SMEM))) return rc;
     attn_fwd_tm_kernel<<<grid, kTcThreads, fwd2::SMEM, stream>>>(mq, mk, mv, p);
     return msamp_check_launch("attn_fwd_tm_kernel");
   }
-  const int n_items = n_qt * batch * heads;
-  const int ctas = n_items < msamp_sm_count() ? n_items : msamp_sm_count();
+  if (kind == SPLIT) {
+    if ((rc = set_smem(attn_fwd_split_kernel, fwd2s::SMEM3))) return rc;
+    attn_fwd_split_kernel<<<ctas, kTcThreads, fwd2s::SMEM3, stream>>>(mq, mk, mv, p, n_qt, n_items);
+    return msamp_check_launch("attn_fwd_split_kernel");
+  }
   if (head_dim == 128) {
     if ((rc = set_smem(attn_fwd_ps_kernel<128>, fwd3::Cfg<128>::SMEM))) return rc;
     attn_fwd_ps_kernel<128><<<ctas, kPsThreads, fwd3::Cfg<128>::SMEM, stream>>>(mq, mk, mv, p, n_qt, n_items);

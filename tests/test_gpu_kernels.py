@@ -564,8 +564,8 @@ def test_gelu():
     assert (x.grad.float() - xr.grad).abs().max().item() <= 3e-2
 
 
-def _attn_ref(q, k, v, causal):
-    qf, kf, vf = (t.float().permute(0, 2, 1, 3) for t in (q, k, v))
+def _attn_ref(q, k, v, causal, dtype=torch.float32):
+    qf, kf, vf = (t.to(dtype).permute(0, 2, 1, 3) for t in (q, k, v))
     s = (qf @ kf.transpose(-1, -2)) / math.sqrt(q.shape[-1])
     if causal:
         S = q.shape[1]
@@ -733,6 +733,24 @@ def test_attention_repeated_heads(d):
     assert _rel(o, r) <= 2 * 2**-9
     for got, ref in zip((q, k, v), leaves):
         assert _rel(got.grad, ref.grad) <= 3 * 2**-9
+
+
+# every forward kernel: (rows, heads) -> one CTA per tile, a list of short rows, both streams of a CTA on one item, a stream per item
+@pytest.mark.parametrize('d, S, H', [(64, 200, 3), (64, 200, 512), (64, 600, 3), (128, 100, 3), (128, 100, 300), (128, 500, 3), (128, 500, 80)])
+def test_attention_largest_probability_is_exact(d, S, H):
+    """Two keys count, a factor of 139 or 147 apart, the larger in the second half of the keys: the largest probability of a row is
+    taken relative to itself, i.e. 1, and adds no rounding of its own (relative to the first key bf16 holds it to 0.3 %)."""
+    torch.manual_seed(4)
+    q, k = torch.zeros(2, 1, S, H, d, device=DEV)
+    q[..., 0] = 1.0
+    k[..., 0] = -40 * math.log(2) * math.sqrt(d)
+    k[:, 5, :, 0] = 0
+    k[:, S - 20, :, 0] = 39.5 if d == 64 else 56.5    # scores 4.94 and 4.99
+    qkv = torch.stack([q, k, torch.randn_like(q)], 2).bfloat16()
+    o = K.attention_qkv(qkv, causal=False)
+    r = _attn_ref(*(qkv[:, :, i].double() for i in range(3)), False, dtype=torch.float64)
+    # one rounding of the output to bf16 (at most 2^-9 of each value) and of the small probability (2^-9 of 2^-7 of V)
+    assert _rel(o, r) <= 2**-9 * (1 + 2**-6)
 
 
 @pytest.mark.parametrize('d', [64, 128])
