@@ -1,5 +1,6 @@
 // Causal (or full) softmax attention, forward and backward, for bf16 with head size 64 or 128, on mma.sync: the path of views
-// with a zero stride (repeated heads), which the tensor maps of attention_tc.cu cannot describe, and a cross-check of it.
+// with a zero stride (repeated heads), which the tensor maps of attention_tc.cu cannot describe, and of short rows, where they are
+// faster (see short_rows there); elsewhere a cross-check of it.
 //
 // Flash-style tiling: a CTA of four warps owns 64 query rows (forward and dQ) or 64 key rows
 // (dK/dV); the other operand streams through shared memory in 64- or 32-row tiles with cp.async

@@ -19,7 +19,7 @@
 //
 // Head size 64 took the mma.sync kernels of attention.cu before: 8 x 1024 x 12 heads, causal, 71 + 253 us forward + backward on
 // the device, now 44 + 107 us; 64 x 197 x 12 heads, 61 + 218 us, now 45 + 119 us.  Those kernels remain for views that a tensor map
-// cannot describe and as a cross-check (MSAMP_ATTN_IMPL=mma).
+// cannot describe, for short rows (see short_rows) and as a cross-check (MSAMP_ATTN_IMPL=mma).
 #include <cstdlib>
 #include <mutex>
 #include <unordered_map>
@@ -3436,6 +3436,35 @@ static bool has_repeats(const int64_t* strides, int tensors, int batch, int head
   return false;
 }
 
+// Short rows: the mma.sync kernels of attention.cu, whose 64-row tiles pad less and whose small CTAs share an SM, where they are the
+// faster ones.  tcgen05 time over mma.sync time, causal / full, at heads * batch = 12, 96 and 768:
+//   head  rows      forward                          backward
+//   64    16        2.0/2.0  2.1/2.1  2.1/2.1        1.8/1.7  1.7/1.7  2.4/2.4
+//   64    64        1.9/2.0  1.9/2.2  1.9/2.0        1.4/1.4  1.4/1.3  1.5/1.4
+//   64    128       1.8/1.6  1.4/1.4  1.0/0.8        1.1/1.1  0.8/0.8  0.8/0.6
+//   64    129       1.4/1.5  1.4/1.4  1.3/1.1        1.2/1.1  1.1/1.2  1.0/0.9
+//   64    256       1.3/1.2  1.0/1.0  0.9/0.7        0.9/0.8  0.6/0.8  0.6/0.5
+//   64    320       1.1/1.2  0.9/0.9  1.0/0.9        0.9/0.8  0.7/0.6  0.7/0.6
+//   64    384       1.1/1.1  0.9/0.8  0.9/0.6        0.8/0.7  0.5/0.4  0.6/0.5
+//   128   16        1.1/1.1  1.1/1.2  1.1/1.1        1.3/1.3  1.3/1.3  1.5/1.5
+//   128   64        1.1/1.2  1.2/1.2  1.1/1.2        1.1/1.1  1.1/1.0  1.1/1.0
+// Above 64 rows the line depends on how many of the persistent kernels' items (128-row tiles) there are for each SM.  Head size 128
+// stays on tcgen05 there: its rows are split into two running maxima, which mma.sync does not do (see kSplitRows).
+static bool short_rows(int seqlen, int head_dim, int64_t heads, bool backward) {
+  if (heads > 65535) return false;    // grid.y of those kernels
+  if (seqlen <= 64) return true;
+  if (head_dim != 64) return false;
+  const int64_t sms = msamp_sm_count(), items = heads * ((seqlen + 127) / 128), waves = (items + sms - 1) / sms;
+  if (backward) {
+    if (seqlen <= 128) return 2 * items <= sms;
+    return seqlen <= 192 && waves <= 2 && 10 * items < 7 * waves * sms;    // SMs that idle in the last wave
+  }
+  if (seqlen <= 128) return items <= 4 * sms;
+  if (seqlen <= 192) return true;    // three 64-row tiles against two of 128
+  if (seqlen <= 320) return 2 * items <= 3 * sms;
+  return seqlen <= 384 && 2 * items <= sms;
+}
+
 extern "C" int msamp_attention_fwd(const void*, const void*, const void*, void*, float*, const int64_t*, int, int, int, int, float, int, void*);
 extern "C" int msamp_attention_bwd(const void*, const void*, const void*, const void*, const float*, const void*, void*, void*, void*, float*,
                                    const int64_t*, int, int, int, int, float, int, void*);
@@ -3458,7 +3487,7 @@ MSAMP_API int msamp_attention_tc_fwd(const void* q, const void* k, const void* v
   MSAMP_REQUIRE(batch > 0 && heads > 0 && seqlen > 0, "attention: empty problem");
   MSAMP_REQUIRE(aligned16(q) && aligned16(k) && aligned16(v) && aligned16(o), "attention: q, k, v and o must be 16-byte aligned");
   for (int i = 0; i < 12; ++i) MSAMP_REQUIRE(strides[i] % 8 == 0, "attention: stride %d is not a multiple of 8 elements", i);
-  if (has_repeats(strides, 3, batch, heads, seqlen))
+  if (has_repeats(strides, 3, batch, heads, seqlen) || short_rows(seqlen, head_dim, (int64_t)batch * heads, false))
     return msamp_attention_fwd(q, k, v, o, lse, strides, batch, heads, seqlen, head_dim, scale, causal, stream_);
   // MSAMP_ATTN_FWD_SMEM=1 selects the kernel with 64-key score tiles and P in shared memory (default: 128-key score
   // tiles, P in tensor memory), MSAMP_ATTN_FWD_PERSIST=0 one CTA per (query tile, batch, head) instead of persistent CTAs.
@@ -3521,7 +3550,7 @@ MSAMP_API int msamp_attention_tc_bwd(const void* q, const void* k, const void* v
   MSAMP_REQUIRE(aligned16(q) && aligned16(k) && aligned16(v) && aligned16(o) && aligned16(d_o) && aligned16(dq) && aligned16(dk) && aligned16(dv),
                 "attention: q, k, v, o, dO and the gradients must be 16-byte aligned");
   for (int i = 0; i < 24; ++i) MSAMP_REQUIRE(strides[i] % 8 == 0, "attention: stride %d is not a multiple of 8 elements", i);
-  if (has_repeats(strides, 5, batch, heads, seqlen))
+  if (has_repeats(strides, 5, batch, heads, seqlen) || short_rows(seqlen, head_dim, (int64_t)batch * heads, true))
     return msamp_attention_bwd(q, k, v, o, lse, d_o, dq, dk, dv, delta, strides, batch, heads, seqlen, head_dim, scale, causal, stream_);
   // MSAMP_ATTN_BWD_SMEM=1 selects the kernels with 64-wide score tiles and the second operand in shared memory,
   // MSAMP_ATTN_BWD_PERSIST=0 one CTA per (tile, batch, head) instead of persistent CTAs over the work items

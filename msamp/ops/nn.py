@@ -191,8 +191,8 @@ def gelu(x):
 
 # ---------------------------------------------------------------------------------------- attention
 def _attn_entry(which):
-    """Native entry point: the tcgen05 kernels (``MSAMP_ATTN_IMPL=mma`` selects the mma.sync kernels, which also serve views
-    with a zero stride)."""
+    """Native entry point: the tcgen05 kernels (``MSAMP_ATTN_IMPL=mma`` selects the mma.sync kernels, to which this entry also
+    sends views with a zero stride and short rows)."""
     tc = os.environ.get('MSAMP_ATTN_IMPL', 'tc') != 'mma'
     return getattr(native.lib(), f'msamp_attention_{"tc_" if tc else ""}{which}')
 

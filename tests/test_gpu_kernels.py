@@ -735,6 +735,37 @@ def test_attention_repeated_heads(d):
         assert _rel(got.grad, ref.grad) <= 3 * 2**-9
 
 
+def _route_cases():
+    """(head size, rows, heads, forward on mma.sync, backward on mma.sync) on both sides of every line of the rule."""
+    sms = native.lib().msamp_device_sm_count() if torch.cuda.is_available() else 148
+    yield from ((64, 64, 5, True, True), (128, 64, 5, True, True), (128, 65, 5, False, False), (64, 64, 2 * sms, True, True))
+    yield from ((64, 65, sms // 2, True, True), (64, 128, sms // 2 + 1, True, False), (64, 128, 4 * sms, True, False), (64, 128, 4 * sms + 1, False, False))
+    yield from ((64, 129, sms // 3, True, True), (64, 192, sms // 2, True, False), (64, 192, sms // 2 + 8, True, True), (64, 192, sms, True, False))
+    yield from ((64, 193, 3 * sms // 4, True, False), (64, 193, 3 * sms // 4 + 1, False, False), (64, 321, sms // 6, True, False), (64, 321, sms // 6 + 1, False, False))
+    yield from ((64, 385, 1, False, False), )
+
+
+@pytest.mark.parametrize('d, S, H, fwd_mma, bwd_mma', list(_route_cases()))
+def test_attention_route_of_short_rows(d, S, H, fwd_mma, bwd_mma, monkeypatch):
+    """The rule by rows and heads, seen by the bits (above 64 rows the two families round differently), and every mixture of
+    families in forward and backward against fp32."""
+    torch.manual_seed(6)
+    qkv = torch.randn(1, S, 3, H, d, device=DEV, dtype=torch.bfloat16)
+    do = torch.randn(1, S, H, d, device=DEV, dtype=torch.bfloat16)
+    o, lse = K.attention_qkv_fwd_raw(qkv, True)
+    g = K.attention_qkv_bwd_raw(qkv, o, lse, do, True)
+    monkeypatch.setenv('MSAMP_ATTN_IMPL', 'mma')
+    o_mma, _ = K.attention_qkv_fwd_raw(qkv, True)
+    g_mma = K.attention_qkv_bwd_raw(qkv, o, lse, do, True)
+    assert torch.equal(o, o_mma) == fwd_mma and torch.equal(g, g_mma) == bwd_mma
+    ref = qkv.detach().float().requires_grad_()
+    r = _attn_ref(ref[:, :, 0], ref[:, :, 1], ref[:, :, 2], True)
+    r.backward(do.float())
+    # bf16 roundings of 2^-9: P and the output forward; P or dS, the saved output and the gradient backward
+    assert _rel(o, r) <= 2 * 2**-9 and _rel(g, ref.grad) <= 3 * 2**-9
+    assert native.device_status() == 0
+
+
 # every forward kernel: (rows, heads) -> one CTA per tile, a list of short rows, both streams of a CTA on one item, a stream per item
 @pytest.mark.parametrize('d, S, H', [(64, 200, 3), (64, 200, 512), (64, 600, 3), (128, 100, 3), (128, 100, 300), (128, 500, 3), (128, 500, 80)])
 def test_attention_largest_probability_is_exact(d, S, H):
