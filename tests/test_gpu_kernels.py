@@ -716,23 +716,158 @@ def test_attention_work_lists(d, shape):
 
 
 @pytest.mark.parametrize('d', [64, 128])
-def test_attention_repeated_heads(d):
+@pytest.mark.parametrize('S', [1, 63, 64, 129, 200])
+@pytest.mark.parametrize('causal', [True, False])
+def test_attention_repeated_heads(d, S, causal):
     """Views with a zero stride (one K / V head for all query heads), which no tensor map can describe."""
     torch.manual_seed(2)
-    B, S, H = 2, 200, 4
+    B, H = 2, 4
     q = torch.randn(B, S, H, d, device=DEV, dtype=torch.bfloat16).requires_grad_()
     kv = torch.randn(2, B, S, 1, d, device=DEV, dtype=torch.bfloat16)
     k, v = (t.expand(B, S, H, d).detach().requires_grad_() for t in kv)
     assert k.stride(2) == 0
-    o = K.attention(q, k, v, causal=True)
+    o = K.attention(q, k, v, causal=causal)
     do = torch.randn_like(o)
     o.backward(do)
     leaves = [t.detach().float().requires_grad_() for t in (q, k, v)]
-    r = _attn_ref(*leaves, True)
+    r = _attn_ref(*leaves, causal)
     r.backward(do.float())
     assert _rel(o, r) <= 2 * 2**-9
-    for got, ref in zip((q, k, v), leaves):
+    for got, ref in list(zip((q, k, v), leaves))[2 if S == 1 else 0:]:    # with one key the gradients of q and k are exactly zero
         assert _rel(got.grad, ref.grad) <= 3 * 2**-9
+
+
+@pytest.mark.parametrize('d', [64, 128])
+@pytest.mark.parametrize('S', [1, 63, 64, 65, 129, 320])
+@pytest.mark.parametrize('causal', [True, False])
+def test_attention_mma_sync_kernels(d, S, causal, monkeypatch):
+    """The path of zero-stride views and short rows, at its tile edges (64 rows forward and dQ, 64 x 32 in dK / dV)."""
+    monkeypatch.setenv('MSAMP_ATTN_IMPL', 'mma')
+    torch.manual_seed(7)
+    qkv = torch.randn(2, S, 3, 3, d, device=DEV, dtype=torch.bfloat16)
+    do = torch.randn(2, S, 3, d, device=DEV, dtype=torch.bfloat16)
+    o, g = _attention_grads(qkv, causal, do)
+    ref = qkv.float().requires_grad_()
+    r = _attn_ref(ref[:, :, 0], ref[:, :, 1], ref[:, :, 2], causal)
+    r.backward(do.float())
+    assert _rel(o, r) <= 2 * 2**-9
+    if S > 1:
+        assert _rel(g, ref.grad) <= 3 * 2**-9
+
+
+@pytest.mark.parametrize('d', [64, 128])
+@pytest.mark.parametrize('S', [70, 500])
+def test_attention_gradient_views(d, S):
+    """Output gradients with other strides: read in place (permuted), copied (rows of an odd length), or repeated over the batch or the
+    heads, which sends a backward to mma.sync whose forward may have run on tcgen05."""
+    torch.manual_seed(8)
+    B, H = 2, 3
+    qkv = torch.randn(B, S, 3, H, d, device=DEV, dtype=torch.bfloat16)
+    full = torch.randn(B, S, H, d, device=DEV, dtype=torch.bfloat16)
+    _, want = _attention_grads(qkv, True, full)
+    permuted = full.permute(0, 2, 1, 3).contiguous().permute(0, 2, 1, 3)
+    wide = torch.zeros(B, S, H, d + 4, device=DEV, dtype=torch.bfloat16)
+    wide[..., :d] = full
+    for do in (permuted, wide[..., :d]):
+        assert not do.is_contiguous() and torch.equal(_attention_grads(qkv, True, do)[1], want)
+    for one in (full[:1], full[:, :, :1]):
+        do = one.expand(B, S, H, d)
+        got, want = (_attention_grads(qkv, True, t)[1] for t in (do, do.contiguous()))
+        assert _rel(got, want) <= 3 * 2**-9    # two families: roundings of P or dS and of the gradient
+
+
+@pytest.mark.parametrize('d', [64, 128])
+def test_attention_saved_tensors_in_other_layouts(d):
+    """Saved-tensor hooks may hand back other strides or an address that is not 16-byte aligned."""
+    torch.manual_seed(9)
+    B, S, H = 2, 260, 3
+    qkv = torch.randn(B, S, 3, H, d, device=DEV, dtype=torch.bfloat16)
+    do = torch.randn(B, S, H, d, device=DEV, dtype=torch.bfloat16)
+    _, want = _attention_grads(qkv, True, do)
+
+    def moved(t):
+        if t.dtype != torch.bfloat16:
+            return t
+        if t.dim() == 5:
+            return t.permute(2, 0, 1, 3, 4).contiguous().permute(1, 2, 0, 3, 4)
+        buf = torch.empty(t.numel() + 4, dtype=t.dtype, device=t.device)
+        buf[4:] = t.flatten()
+        return buf[4:].view(t.shape)
+
+    leaf = qkv.clone().requires_grad_()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, moved):
+        K.attention_qkv(leaf, causal=True).backward(do)
+    assert torch.equal(leaf.grad, want)
+
+
+# two running maxima per row (64) or one (128); both streams of a CTA on one item (20 items), or a stream per item and a shared last wave
+@pytest.mark.parametrize('d', [64, 128])
+@pytest.mark.parametrize('H', [2, 40])
+def test_attention_growing_maximum(d, H, monkeypatch):
+    """Scores that grow along the keys: the accumulators are rescaled in most tiles."""
+    torch.manual_seed(1)
+    B, S = 1, 1280
+    qkv = torch.randn(B, S, 3, H, d, device=DEV)
+    qkv[:, :, 1] *= torch.linspace(0.2, 6.0, S, device=DEV).view(1, S, 1, 1)
+    qkv = qkv.bfloat16()
+    do = torch.randn(B, S, H, d, device=DEV, dtype=torch.bfloat16)
+    o, g = _attention_grads(qkv, True, do)
+    ref = qkv.float().requires_grad_()
+    r = _attn_ref(ref[:, :, 0], ref[:, :, 1], ref[:, :, 2], True)
+    r.backward(do.float())
+    assert _rel(o, r) <= 2 * 2**-9
+    assert native.device_status() == 0
+    # the gradients of peaked rows depend on how far dP and delta cancel: the other family's error is the measure
+    monkeypatch.setenv('MSAMP_ATTN_IMPL', 'mma')
+    o_mma, g_mma = _attention_grads(qkv, True, do)
+    ratio = _rel(o, r) / _rel(o_mma, r)
+    assert ratio <= 1.02 or d == 128    # from the fifth tile of 128 keys on, head size 128 lets the maximum lag (bounded above)
+    assert _rel(g, ref.grad) <= 1.05 * max(1.0, ratio) * _rel(g_mma, ref.grad)    # delta inherits the error of the saved output
+
+
+# more than two waves of both streams (downward waves) and more heads than a group of the work order holds
+@pytest.mark.parametrize('d, H, causal', [(64, 320, True), (64, 320, False), (128, 160, True), (128, 160, False)])
+def test_attention_several_groups_of_heads(d, H, causal):
+    torch.manual_seed(10)
+    S = 640
+    assert H * S * d * 4 > 48 << 20 and 5 * H > 4 * native.lib().msamp_device_sm_count()
+    qkv = torch.randn(1, S, 3, H, d, device=DEV, dtype=torch.bfloat16)
+    do = torch.randn(1, S, H, d, device=DEV, dtype=torch.bfloat16)
+    o, g = _attention_grads(qkv, causal, do)
+    ref = qkv.float().requires_grad_()
+    r = _attn_ref(ref[:, :, 0], ref[:, :, 1], ref[:, :, 2], causal)
+    r.backward(do.float())
+    for h in range(H):    # each head by itself, so that a swapped or skipped item shows
+        assert _rel(o[:, :, h], r[:, :, h]) <= 2 * 2**-9 and _rel(g[:, :, :, h], ref.grad[:, :, :, h]) <= 3 * 2**-9, h
+    assert native.device_status() == 0
+
+
+@pytest.mark.parametrize('impl', ['tc', 'mma'])
+@pytest.mark.parametrize('d', [64, 128])
+@pytest.mark.parametrize('S', [200, 700])
+@pytest.mark.parametrize('bad', [float('nan'), float('inf')])
+def test_attention_not_finite_rows(impl, d, S, bad, monkeypatch):
+    """A query with NaN, or whose scores reach infinity, gives a NaN row; the other rows and their gradients are as without it."""
+    monkeypatch.setenv('MSAMP_ATTN_IMPL', impl)
+    torch.manual_seed(11)
+    H, row = 2, S - 30
+    qkv = torch.randn(1, S, 3, H, d, device=DEV, dtype=torch.bfloat16)
+    do = torch.randn(1, S, H, d, device=DEV, dtype=torch.bfloat16)
+    o, g = _attention_grads(qkv, False, do)
+    qkv[0, row, 0, 1, 0] = bad
+    o2, g2 = _attention_grads(qkv, False, do)
+    others = [i for i in range(S) if i != row]
+    assert o2[0, row, 1].isnan().all() and not g2[0, row, 0, 1].isfinite().any()
+    assert torch.equal(o2[0, others], o[0, others]) and torch.equal(o2[0, row, 0], o[0, row, 0])
+    assert torch.equal(g2[0, others, 0], g[0, others, 0]) and torch.equal(g2[:, :, :, 0], g[:, :, :, 0])
+    assert native.device_status() == 0
+
+
+def _attention_grads(qkv, causal, do):
+    leaf = qkv.detach().clone().requires_grad_()
+    o = K.attention_qkv(leaf, causal=causal)
+    o.backward(do)
+    return o.detach(), leaf.grad
 
 
 def _route_cases():
