@@ -72,6 +72,7 @@ __device__ __forceinline__ float st_max(int st) {
 struct Raw8 {
   Bytes16 a, b;
 };
+constexpr int raw_regs(int st) { return st == ST_F32 ? 8 : (st == ST_F16 || st == ST_BF16 ? 4 : 2); }    // of eight stored elements
 __device__ __forceinline__ Raw8 load8_raw(const void* base, int st, int64_t i) {
   Raw8 r;
   switch (st) {
@@ -316,8 +317,10 @@ __device__ __forceinline__ void adam_block(AdamTensor& t, int64_t begin, int64_t
       }
     };
     // U steps' loads are issued before the first of them is used: the compiler may not move a load of the next step over the
-    // stores of this one
-    constexpr int U = PS < 0 ? 1 : (MS == ST_F32 ? 2 : 4);
+    // stores of this one.  Four steps where they take at most 56 registers, else two (four fp32 steps of a parameter and its
+    // gradient spilled: 238 -> 228 us for 50 M parameters at f32/f32/e4m3/f16); two where the codes are read at run time
+    // (318 -> 262 us at f32/bf16/f16/f16 against one).
+    constexpr int U = PS >= 0 && raw_regs(PS) + raw_regs(GS) + raw_regs(MS) + raw_regs(VS) <= 14 ? 4 : 2;
     constexpr int64_t step = (int64_t)kAdamThreads * 8;
     int64_t i = begin + (int64_t)threadIdx.x * 8;
     for (; i + (U - 1) * step + 8 <= end; i += U * step) {
@@ -447,7 +450,9 @@ __device__ __forceinline__ void adam_block_reduce(AdamTensor& t, const PeerGrads
   }
 }
 
-__global__ void __launch_bounds__(kAdamThreads) lbadam_reduce_stage1_kernel(AdamTensor* tensors, const int* __restrict__ work, const PeerGrads pg) {
+// Three CTAs per SM: it waits for loads over NVLink.  Left to itself the compiler takes 127 registers (two CTAs); one rank, 50 M
+// parameters, both stages: 345 us then, 282 with three, 316 before the f32x2 loop.
+__global__ void __launch_bounds__(kAdamThreads, 3) lbadam_reduce_stage1_kernel(AdamTensor* tensors, const int* __restrict__ work, const PeerGrads pg) {
   __shared__ float red[32];
   AdamTensor& t = tensors[work[2 * blockIdx.x]];
   const int chunk = work[2 * blockIdx.x + 1];
