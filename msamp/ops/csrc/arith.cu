@@ -147,7 +147,7 @@ MSAMP_API int msamp_add_to_fp8(void* fp8, int64_t n, int fmt, float* scale, floa
   if (n == 0) return MSAMP_OK;
   cudaMemsetAsync(amax_tmp, 0, sizeof(float), stream);
   const bool vec = (reinterpret_cast<uintptr_t>(fp8) & 7) == 0 && (reinterpret_cast<uintptr_t>(other) & 15) == 0;
-  int grid = msamp_grid_for(vec ? (n + 15) / 16 : n, kThreads, 6);
+  int grid = msamp_grid_for(vec ? (n + 15) / 16 : n, kThreads, vec ? 6 : 8);    // byte by byte: 13 M elements 39.1 -> 37.5 us with eight
 #define MSAMP_ADD_LAUNCH(V)                                                                                                           \
   {                                                                                                                                   \
     add_amax_kernel<T, F, V><<<grid, kThreads, 0, stream>>>((const uint8_t*)fp8, (const T*)other, n, scale_inv, amax_tmp);              \

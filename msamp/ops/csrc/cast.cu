@@ -492,10 +492,14 @@ MSAMP_API int msamp_amax(const void* x, int64_t n, int dtype, float* amax, float
   cudaStream_t stream = (cudaStream_t)stream_;
   MSAMP_REQUIRE(n >= 0 && amax != nullptr, "msamp_amax: bad arguments");
   cudaMemsetAsync(amax, 0, sizeof(float), stream);
-  int grid = msamp_grid_for((n + 63) / 64, kThreads, 4);
-  if (n == 0) grid = 1;
+  // One pass of a thread takes 8 vectors; 16-bit types want four CTAs per SM, fp32 six (102 MB 17.6 -> 16.6 us, 200 MB 32.0 -> 30.9 us;
+  // the half-empty last pass of larger steps shows there).  Element by element, more and smaller CTAs: 100000 unaligned elements
+  // 8.3 -> 6.4 us, 25.6 M fp32 30.0 -> 22.7 us.
+  const bool vec = aligned16(x);
+  const bool wide = vec && dtype != DT_F32;
+  const int grid = n == 0 ? 1 : msamp_grid_for(wide ? (n + 63) / 64 : (n + 31) / 32, kThreads, wide ? 4 : 6);
   MSAMP_DISPATCH_HP(dtype, T, {
-    if (aligned16(x))
+    if (vec)
       amax_kernel<T, true><<<grid, kThreads, 0, stream>>>((const T*)x, n, amax, scale, scale_inv, fp_max, margin, prescale, counter);
     else
       amax_kernel<T, false><<<grid, kThreads, 0, stream>>>((const T*)x, n, amax, scale, scale_inv, fp_max, margin, prescale, counter);
