@@ -161,19 +161,21 @@ __global__ void __launch_bounds__(kThreads) cast_to_fp8_kernel(const T* __restri
 // ---- high precision [rows, cols] -> fp8 with the column sums of the input -------------------------
 // Used for the output gradient of a linear layer: the bias gradient falls out of the pass that
 // quantises dy.  Memory bound.  A CTA owns a slab of 32 16-byte column vectors (512 bytes of a row, one per lane) and a range
-// of rows that its eight warps take in turn, kColsumRows in flight per thread.  Every thread keeps the partial sums of its own
+// of rows that its eight warps take in turn, U in flight per thread.  Every thread keeps the partial sums of its own
 // columns in registers; the warps are combined in shared memory and the CTA adds one value per column to colsum (fp32, zeroed
 // by the caller).  One CTA row per 256 vectors with eight strided atomics per thread spent most of its time in them:
-// 8192 x 4096 bf16 60 -> 24 us, 1576 x 3072 33 -> 6.6 us.  cols must be a multiple of 16 bytes.
-constexpr int kColsumRows = 8;    // rows in flight per thread
+// 8192 x 4096 bf16 55 -> 21 us, 1576 x 3072 39 -> 8.4 us, 4096 x 16384 fp32 57 -> 55 us.  Four CTAs are resident per SM (64
+// registers) and the grid is no larger than that: with 70 registers and one row of CTAs more, 4096 x 16384 fp32 took 64 us.  Plain
+// loads: streaming ones cost 8192 x 16384 fp32 9 % (113 against 103 us).  cols must be a multiple of 16 bytes.
+constexpr int kColsumRows = 8;       // rows in flight per thread, and
+constexpr int kColsumFewRows = 2;    // where a warp has at most four: the eight-row code costs calls of some 5 us up to 1.3 us
 constexpr int kColsumWarps = kThreads / 32;
-template <typename T, int FMT>
-__global__ void __launch_bounds__(kThreads) cast_rows_colsum_kernel(const T* __restrict__ x, uint8_t* __restrict__ out, int rows, int cols,
+template <typename T, int FMT, int U>
+__global__ void __launch_bounds__(kThreads, 4) cast_rows_colsum_kernel(const T* __restrict__ x, uint8_t* __restrict__ out, int rows, int cols,
                                                                      int rows_per_cta, float* scale_ptr, float* amax, float* scale_inv_out,
                                                                      float* __restrict__ colsum, const float* amax_in, float fp_max) {
   __shared__ float red[32];
   constexpr int N = VecOf<T>::N;
-  constexpr int U = kColsumRows;
   __shared__ float part[kColsumWarps][33 * N];
   float scale = *scale_ptr;
   if (amax_in != nullptr) {    // in-time scaling from an amax that the producer of x already reduced
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(kThreads) cast_rows_colsum_kernel(const T* __r
       Bytes16 v[U];
 #pragma unroll
       for (int u = 0; u < U; ++u)
-        if (r + u * kColsumWarps < r1) v[u] = ld_stream16(xv + (int64_t)(r + u * kColsumWarps) * cv);
+        if (r + u * kColsumWarps < r1) v[u] = xv[(int64_t)(r + u * kColsumWarps) * cv];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int rr = r + u * kColsumWarps;
@@ -554,16 +556,20 @@ MSAMP_API int msamp_cast_to_fp8_colsum(const void* x, int rows, int cols, int dt
   if (amax) cudaMemsetAsync(amax, 0, sizeof(float), stream);
   if ((int64_t)rows * cols == 0) return MSAMP_OK;
   const int slabs = (cols * esize / 16 + 31) / 32;
-  // four CTAs per SM if the rows give every thread at least one full load batch, else as many as they give half a batch
-  int chunks = (msamp_sm_count() * 4 + slabs - 1) / slabs;
-  const int most = (rows + kColsumWarps * kColsumRows / 2 - 1) / (kColsumWarps * kColsumRows / 2);
+  // what is resident at once, and at least two rows for each warp
+  int chunks = msamp_sm_count() * 4 / slabs;
+  const int most = (rows + 2 * kColsumWarps - 1) / (2 * kColsumWarps);
   if (chunks > most) chunks = most;
+  if (chunks < 1) chunks = 1;
   const int rows_per_cta = (rows + chunks - 1) / chunks;
-  chunks = (rows + rows_per_cta - 1) / rows_per_cta;    // <= 65535: chunks <= 4 * SMs + 1
+  chunks = (rows + rows_per_cta - 1) / rows_per_cta;    // <= 65535: chunks <= 4 * SMs
   dim3 grid((unsigned)slabs, (unsigned)chunks, 1);
   MSAMP_DISPATCH_HP(dtype, T, {
     MSAMP_DISPATCH_FP8(fmt, F, {
-      cast_rows_colsum_kernel<T, F><<<grid, kThreads, 0, stream>>>((const T*)x, (uint8_t*)out, rows, cols, rows_per_cta, scale, amax, scale_inv_out, colsum, amax_in, fp8_max(F));
+      if (rows_per_cta <= 4 * kColsumWarps)
+        cast_rows_colsum_kernel<T, F, kColsumFewRows><<<grid, kThreads, 0, stream>>>((const T*)x, (uint8_t*)out, rows, cols, rows_per_cta, scale, amax, scale_inv_out, colsum, amax_in, fp8_max(F));
+      else
+        cast_rows_colsum_kernel<T, F, kColsumRows><<<grid, kThreads, 0, stream>>>((const T*)x, (uint8_t*)out, rows, cols, rows_per_cta, scale, amax, scale_inv_out, colsum, amax_in, fp8_max(F));
     });
   });
   return msamp_check_launch("msamp_cast_to_fp8_colsum");

@@ -308,7 +308,8 @@ def test_add_to_fp8_vector_edges(n, offset):
         assert t.meta.scale.item() == c.meta.scale.item() and t.meta.amax[0].item() == c.meta.amax[0].item()
 
 
-@pytest.mark.parametrize('shape', [(1, 8), (31, 248), (33, 264), (257, 256), (1576, 3072), (5000, 40)])    # rows per CTA, column slabs of 256
+# column slabs of 512 bytes, two or eight rows in flight (up to 32 rows per CTA, more), last chunks that are short
+@pytest.mark.parametrize('shape', [(1, 8), (31, 248), (33, 264), (257, 256), (1576, 3072), (5000, 40), (2048, 4096), (2047, 8200)])
 @pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
 def test_cast_colsum_slabs(shape, dtype):
     torch.manual_seed(0)
