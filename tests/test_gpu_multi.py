@@ -253,7 +253,8 @@ def _zero2_training(rank, world, fuse_adam=True, overlap=False):
 
 def _fused_adam_equals_reduce_then_adam(rank, world):
     """One optimizer step from the same gradients and states, once with the reduce-scatter folded into the Adam kernel and
-    once with the separate reduce kernel: masters, moments and published FP8 weights agree bit for bit."""
+    once with the separate reduce kernel: masters, moments, their scales and maxima and published FP8 weights agree bit for bit.
+    A first step fills the moments, so that both start from the same non-zero ones."""
     from msamp.ops import native
     from msamp.parallel.zero import ZeroShardedOptimizer
     dev = torch.device('cuda', rank)
@@ -271,19 +272,32 @@ def _fused_adam_equals_reduce_then_adam(rank, world):
                 masters={i: (m.value.clone(), m.meta.scale.clone(), m.meta.scale_inv.clone(), m.meta.amax.clone()) for i, m in zero.masters.items()},
                 hp=[p.detach().clone() for p in zero.hp_params], hp_grads=[None if p.grad is None else p.grad.clone() for p in zero.hp_params],
                 fp8_grads=[p.grad for p in zero.fp8_params])
-    results = []
-    for fused in (True, False):
-        zero.fuse_adam = fused
+    results, moments = [], None
+
+    def parts(t):
+        return (t.value, t.meta.scale, t.meta.scale_inv, t.meta.amax) if hasattr(t, 'meta') else (t, )
+
+    for fused in (None, True, False):
+        zero.fuse_adam = fused is not False
         zero.reduce_and_step()
         torch.cuda.synchronize()
         assert native.device_status() == 0
         dist.barrier()
-        results.append(dict(w=zero.w_flat.clone(), wm=zero.w_meta_t[:2].clone(),
-                            masters={i: m.value.clone() for i, m in zero.masters.items()},
-                            m={i: opt.state[m]['exp_avg'].value.clone() for i, m in zero.masters.items()},
-                            v={i: opt.state[m]['exp_avg_sq'].value.clone() for i, m in zero.masters.items()}))
-        # back to the state before the step
-        opt.state.clear()
+        if fused is None:
+            moments = {p: {k: v if k == 'step' else [t.clone() for t in parts(v)] for k, v in st.items()} for p, st in opt.state.items()}
+        else:
+            results.append(dict(w=zero.w_flat.clone(), wm=zero.w_meta_t[:2].clone(),
+                                masters={i: [t.clone() for t in parts(m)] for i, m in zero.masters.items()},
+                                m={i: [t.clone() for t in parts(opt.state[m]['exp_avg'])] for i, m in zero.masters.items()},
+                                v={i: [t.clone() for t in parts(opt.state[m]['exp_avg_sq'])] for i, m in zero.masters.items()}))
+        # back to the state before the step, with the moments of the first one
+        for p, st in moments.items():
+            for k, saved in st.items():
+                if k == 'step':
+                    opt.state[p][k] = saved
+                else:
+                    for t, old in zip(parts(opt.state[p][k]), saved):
+                        t.copy_(old)
         zero.g_flat.copy_(snap['g'])
         zero.g_meta_t.copy_(snap['gm'])
         zero.w_flat.copy_(snap['w'])
@@ -304,7 +318,8 @@ def _fused_adam_equals_reduce_then_adam(rank, world):
     a, b = results
     assert torch.equal(a['w'], b['w']) and torch.equal(a['wm'], b['wm'])
     for i in a['masters']:
-        assert torch.equal(a['masters'][i], b['masters'][i]) and torch.equal(a['m'][i], b['m'][i]) and torch.equal(a['v'][i], b['v'][i])
+        for kind in ('masters', 'm', 'v'):
+            assert all(torch.equal(x, y) for x, y in zip(a[kind][i], b[kind][i])), (kind, i)
     zero.close()
 
 
