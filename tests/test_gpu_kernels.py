@@ -484,9 +484,10 @@ def test_layernorm(dt, shape):
 
 
 @pytest.mark.parametrize('dt', [torch.bfloat16, torch.float16, torch.float32])
-@pytest.mark.parametrize('rows', [1183, 1184, 5001])    # around the row count from which one warp takes a row (8 per SM)
-@pytest.mark.parametrize('vecs', [1, 31, 33, 95, 129, 257, 511, 512])    # 16-byte vectors per row: edges of the vectors per lane
-def test_layernorm_forward_rows_per_warp(dt, rows, vecs):
+@pytest.mark.parametrize('rows', [7, 5001])    # fewer rows than CTAs, several per CTA
+@pytest.mark.parametrize('vecs', [1, 129, 512, 513])    # 16-byte vectors per row: a CTA has 128 threads of up to four, from 513 on 256
+def test_layernorm_forward_values(dt, rows, vecs):
+    """Output, statistics and maximum against 64 bits, for parameters in fp32 and in the type of the input."""
     torch.manual_seed(0)
     cols = vecs * (4 if dt == torch.float32 else 8)
     x = (torch.randn(rows, cols, device=DEV) * 2 + 0.5).to(dt)
