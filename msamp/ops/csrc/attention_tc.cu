@@ -2923,7 +2923,7 @@ struct Cfg {
   static constexpr int B_KV = 0, B_QF = 1, B_QE = B_QF + NQ, B_OF = B_QE + NQ, B_OE = B_OF + ND, B_SF = B_OE + ND, B_SE = B_SF + 1, B_DF = B_SE + 1,
                        B_PF = B_DF + NB, B_PP = B_PF + NB, B_PE = B_PP + NB, B_ACC = B_PE + NB, B3_KVE = B_ACC + 1, B3_OE = B3_KVE + 1,
                        NBAR = B3_OE + 1;
-  static constexpr int SMEM = OFF_BAR + NBAR * 8 + 16;    // head size 128: 152 bytes below the limit, so the base has to be aligned
+  static constexpr int SMEM = OFF_BAR + NBAR * 8 + 16;    // head size 128: 848 bytes below the limit, so the base has to be aligned
   static constexpr uint32_t TM_ST = 0, TM_DPT = 128, TM_DV = TM_DPT + NB * 128, TM_DK = TM_DV + D, TM_COLS = 512;
   static_assert(SMEM <= 227 * 1024, "persistent dK/dV kernel: shared memory");
   static_assert(TM_DK + D <= TM_COLS, "persistent dK/dV kernel: tensor memory");

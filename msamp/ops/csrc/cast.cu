@@ -24,7 +24,8 @@ __global__ void __launch_bounds__(kThreads) amax_kernel(const T* __restrict__ x,
   if (VEC) {
     // Memory bound once the maximum costs little: |x| as bits is monotone with NaN above inf, so 16-bit elements take two
     // instructions per pair (mask, packed maximum) instead of five per element; eight loads in flight per thread.
-    // 4096 x 50304 bf16 (412 MB) 101 -> 60 us, 4096 x 5120 14.3 -> 10.1 us.
+    // L2 flushed before each call: 4096 x 50304 bf16 (412 MB) 100 -> 72 us (5.7 TB/s), 4096 x 5120 18.5 -> 16.4 us, 103 M fp32 86 ->
+    // 72 us; repeated on the same data, where 126 MB stay in L2, 400 MB take 60 us.
     constexpr int N = VecOf<T>::N;
     constexpr int U = 8;
     int64_t nv = n / N;
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(kThreads) cast_to_fp8_kernel(const T* __restri
 // of rows that its eight warps take in turn, U in flight per thread.  Every thread keeps the partial sums of its own
 // columns in registers; the warps are combined in shared memory and the CTA adds one value per column to colsum (fp32, zeroed
 // by the caller).  One CTA row per 256 vectors with eight strided atomics per thread spent most of its time in them:
-// 8192 x 4096 bf16 55 -> 21 us, 1576 x 3072 39 -> 8.4 us, 4096 x 16384 fp32 57 -> 55 us.  Four CTAs are resident per SM (64
+// repeated calls, 8192 x 4096 bf16 55 -> 21 us (L2 flushed 57 -> 29), 1576 x 3072 39 -> 8.4 us, 4096 x 16384 fp32 57 -> 55 us.  Four CTAs are resident per SM (64
 // registers) and the grid is no larger than that: with 70 registers and one row of CTAs more, 4096 x 16384 fp32 took 64 us.  Plain
 // loads: streaming ones cost 8192 x 16384 fp32 9 % (113 against 103 us).  cols must be a multiple of 16 bytes.
 constexpr int kColsumRows = 8;       // rows in flight per thread, and
@@ -494,8 +495,8 @@ MSAMP_API int msamp_amax(const void* x, int64_t n, int dtype, float* amax, float
   cudaStream_t stream = (cudaStream_t)stream_;
   MSAMP_REQUIRE(n >= 0 && amax != nullptr, "msamp_amax: bad arguments");
   cudaMemsetAsync(amax, 0, sizeof(float), stream);
-  // One pass of a thread takes 8 vectors; 16-bit types want four CTAs per SM, fp32 six (102 MB 17.6 -> 16.6 us, 200 MB 32.0 -> 30.9 us;
-  // the half-empty last pass of larger steps shows there).  Element by element, more and smaller CTAs: 100000 unaligned elements
+  // One pass of a thread takes 8 vectors; 16-bit types want four CTAs per SM, fp32 six (repeated calls on 102 MB 17.6 -> 16.6 us, on
+  // 200 MB 32.0 -> 30.9 us; the half-empty last pass of larger steps shows there).  Element by element, more and smaller CTAs: 100000 unaligned elements
   // 8.3 -> 6.4 us, 25.6 M fp32 30.0 -> 22.7 us.
   const bool vec = aligned16(x);
   const bool wide = vec && dtype != DT_F32;

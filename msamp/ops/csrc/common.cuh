@@ -213,8 +213,8 @@ struct alignas(8) Bytes8 { uint32_t w[2]; };
 
 // Streaming load of data that no thread writes while the kernel runs: not allocated in L1.  A pure read of 412 MB ran at 5.0 TB/s
 // with plain 16-byte loads, whatever their number in flight, their order or their width, and at 5.9 to 6.0 TB/s with these.
-// For reads only: passes that store about as much as they read, or whose data the next pass wants in L2, were up to 20 % slower
-// with them (FP8 casts, cross-entropy, both passes of add_to_fp8, stage 2 of Adam).
+// For reads only (amax): passes that store about as much as they read, or whose data the next pass wants in L2, were up to 20 %
+// slower with them (FP8 casts with and without column sums, cross-entropy, both passes of add_to_fp8, stage 2 of Adam).
 __device__ __forceinline__ Bytes16 ld_stream16(const void* p) {
   Bytes16 r;
   asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]) : "l"(p));

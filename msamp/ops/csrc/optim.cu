@@ -524,7 +524,8 @@ MSAMP_API int msamp_lbadam_chunk() { return kChunk; }
 // `tensors`: device array of n_tensors descriptors (layout of AdamTensor; `red` must be zero on
 // entry); `work`: device array of 2 * n_blocks ints mapping each block to (tensor, chunk).
 // Both stages are bound by memory (O2: 6 bytes read per parameter, then 6 read and 5 written).  One transformer block of hidden
-// size 2048 (50 M parameters): stage 1 86 -> 70 us, stage 2 108 -> 89 us, from f32x2 arithmetic, loads of four steps in flight,
+// size 2048 (50 M parameters): stage 1 86 -> 70 us, stage 2 108 -> 89 us (both 197 -> 155 us in a graph), from f32x2 arithmetic, loads
+// of four steps in flight (stage 2 spills 52 bytes with them at three CTAs per SM; with two steps 164 us, with two CTAs 101 us for it),
 // chunks of 16384 (8192: 85 and 98 us) and stage 2 starting at the end that stage 1 left in L2.  Taking the tensors through
 // both stages in groups that fit L2 was slower (100 and 94 us at 110 MB: the short launches do not fill the GPU).
 MSAMP_API int msamp_lbadam_step(void* tensors, int n_tensors, const int* work, int n_blocks, void* stream_) {
