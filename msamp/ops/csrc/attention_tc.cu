@@ -3455,9 +3455,10 @@ static bool short_rows(int seqlen, int head_dim, int64_t heads, bool backward) {
   if (seqlen <= 64) return true;
   if (head_dim != 64) return false;
   const int64_t sms = msamp_sm_count(), items = heads * ((seqlen + 127) / 128), waves = (items + sms - 1) / sms;
+  const bool idle = waves <= 2 && 10 * items < 7 * waves * sms;    // SMs without an item in the last wave
   if (backward) {
-    if (seqlen <= 128) return 2 * items <= sms;
-    return seqlen <= 192 && waves <= 2 && 10 * items < 7 * waves * sms;    // SMs that idle in the last wave
+    if (seqlen <= 128) return 2 * items <= sms || (idle && waves == 2 && seqlen <= 96);
+    return idle && seqlen <= 192;
   }
   if (seqlen <= 128) return items <= 4 * sms;
   if (seqlen <= 192) return true;    // three 64-row tiles against two of 128

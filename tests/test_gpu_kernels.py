@@ -876,6 +876,7 @@ def _route_cases():
     """(head size, rows, heads, forward on mma.sync, backward on mma.sync) on both sides of every line of the rule."""
     sms = native.lib().msamp_device_sm_count() if torch.cuda.is_available() else 148
     yield from ((64, 64, 5, True, True), (128, 64, 5, True, True), (128, 65, 5, False, False), (64, 64, 2 * sms, True, True))
+    yield from ((64, 96, sms + sms // 4, True, True), (64, 97, sms + sms // 4, True, False), (64, 96, 2 * sms, True, False))
     yield from ((64, 65, sms // 2, True, True), (64, 128, sms // 2 + 1, True, False), (64, 128, 4 * sms, True, False), (64, 128, 4 * sms + 1, False, False))
     yield from ((64, 129, sms // 3, True, True), (64, 192, sms // 2, True, False), (64, 192, sms // 2 + 8, True, True), (64, 192, sms, True, False))
     yield from ((64, 193, 3 * sms // 4, True, False), (64, 193, 3 * sms // 4 + 1, False, False), (64, 321, sms // 6, True, False), (64, 321, sms // 6 + 1, False, False))
