@@ -295,7 +295,8 @@ def test_add_to_fp8_bit_exact():
                 assert t.meta.scale.item() == c.meta.scale.item() and t.meta.amax[0].item() == c.meta.amax[0].item()
 
 
-@pytest.mark.parametrize('n', [7, 8, 9, 16 * 256, 148 * 6 * 256 * 16 + 8 * 256 + 5])    # one vector, its neighbours, one and several grid steps
+# one vector, its neighbours, a CTA, the last size with one step per thread and the next, several grid steps
+@pytest.mark.parametrize('n', [7, 8, 9, 16 * 256, 148 * 4 * 256 * 8, 148 * 4 * 256 * 8 + 1, 148 * 6 * 256 * 16 + 8 * 256 + 5])
 @pytest.mark.parametrize('offset', [0, 1])    # the byte-wise path of unaligned slices
 def test_add_to_fp8_vector_edges(n, offset):
     for dt in (torch.float32, torch.bfloat16):
